@@ -729,18 +729,24 @@ __global__ void k_wrap_psi_lin(const float* __restrict__ psi, const float* __res
 #include "adjoint.cuh"
 
 namespace djb {
-// Kφ as a functor for the fused z pass.
+// Kφ as a functor for the fused z pass: float64 sums and products, one float division
+// (within 1.5 ulp of kphi).
 struct KPhiFn {
     const double* T;
     const double* M;
     double s0;
-    __device__ __forceinline__ float operator()(int kx, int ky, int kz) const { return kphi(T, M, s0, kx, ky, kz); }
-    // float64 sums and products, one float division (within 1.5 ulp of the above)
-    __device__ __forceinline__ float fast(int kx, int ky, int kz) const {
-        if ((kx | ky | kz) == 0) return 0.0f;
-        double num = s0;
-        if (M) num *= M[kx] * M[ky] * M[kz];
-        return float(num) / float(T[kx] + T[ky] + T[kz]);
+    struct Pencil {
+        double t, num;
+        float numf;
+        bool dc;
+    };
+    __device__ __forceinline__ Pencil pencil(int kx, int ky) const {
+        const double num = M ? s0 * (M[kx] * M[ky]) : s0;
+        return Pencil{T[kx] + T[ky], num, float(num), (kx | ky) == 0};
+    }
+    __device__ __forceinline__ float at(const Pencil& p, int kz) const {
+        if (p.dc && kz == 0) return 0.0f;
+        return (M ? float(p.num * __ldg(M + kz)) : p.numf) / float(p.t + __ldg(T + kz));
     }
 };
 }  // namespace djb
@@ -855,8 +861,8 @@ struct djb_solver {
     CUtensorMap tmap_rho;        // the first dense mesh, deposit-box boxes (the VJP's rho-bar gather)
     bool have_tmap_adj = false;
     bool tma = false;
-    // res == 1024: the dense transforms are batched 2-D transforms of the z planes and
-    // the z stages run fused with Kφ in k_zpencil_pair (zpencil.cuh); wN = exp(-2πi j/res)
+    // res 128, 256, 512, 1024: the dense transforms are batched 2-D transforms of the z planes
+    // and the z stages run fused with Kφ in k_zpass (zpencil.cuh); wN = exp(-2πi j/res)
     bool zpass = false;
     float2* wN = nullptr;
     float* adj[3] = {nullptr, nullptr, nullptr};  // VJP work meshes (allocated on first use)
@@ -1293,16 +1299,27 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
 
 // Force evaluation for all shifts; if `step`, fused with the drift/kick/drift.
 // Reads s->psi (and s->mom). Output: s->acc (step == 0) or updated psi/mom.
-// The fused z pass of the 1024³ Poisson solve on the half spectrum in `mesh`.
-void launch_zpass(djb_solver* s, float* mesh, int nh) {
-    const dim3 grid(unsigned((nh + djb::kZPencils - 1) / djb::kZPencils), unsigned(s->res));
-    const djb::KPhiFn kp{s->lapT, s->makT, s->s0};
-    if (DJB_ZPASS_PAIR)
-        djb::k_zpencil_pair<<<grid, djb::kZPairThreads, djb::kZSmem, s->stream>>>(reinterpret_cast<float2*>(mesh), nh,
-                                                                                  s->wN, kp);
-    else
-        djb::k_zpencil_kphi<<<grid, djb::kZThreads, djb::kZSmem, s->stream>>>(reinterpret_cast<float2*>(mesh), nh,
-                                                                              s->wN, kp);
+// The fused z pass of the Poisson solve on the half spectrum in `mesh`.
+template <int N>
+void launch_zpass_n(djb_solver* s, float* mesh) {
+    using G = djb::ZGeom<N>;
+    const dim3 grid(unsigned((N / 2 + djb::kZPencils) / djb::kZPencils), unsigned(N));
+    djb::k_zpass<N><<<grid, G::kThreads, G::kSmem, s->stream>>>(reinterpret_cast<float2*>(mesh), s->wN,
+                                                                djb::KPhiFn{s->lapT, s->makT, s->s0});
+}
+
+void launch_zpass(djb_solver* s, float* mesh) {
+    if (s->res == 128) launch_zpass_n<128>(s, mesh);
+    else if (s->res == 256) launch_zpass_n<256>(s, mesh);
+    else if (s->res == 512) launch_zpass_n<512>(s, mesh);
+    else launch_zpass_n<1024>(s, mesh);
+}
+
+template <int N>
+int zpass_attrs() {
+    CUDA_TRY(cudaFuncSetAttribute(djb::k_zpass<N, djb::KPhiFn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(djb::ZGeom<N>::kSmem)));
+    return DJB_OK;
 }
 
 // Brick sort of the particles at X = q + Ψ (+ dd1·Mom when `mom`): perm (sort.cuh).
@@ -1377,8 +1394,7 @@ int force(djb_solver* s, bool step, double dd1, double alpha, double beta, doubl
             }
             if (s->zpass) {
                 s->prof.begin(s->stream, PH_KSPACE);
-                const int nh = s->res / 2 + 1;
-                launch_zpass(s, mesh, nh);
+                launch_zpass(s, mesh);
                 s->prof.end(s->stream, PH_KSPACE, 1);
                 s->prof.begin(s->stream, PH_C2R);
                 CUFFT_TRY(cufftExecC2R(s->c2r_d, spec, s->phi[m]));
@@ -1464,9 +1480,8 @@ int poisson(djb_solver* s, int m) {
     cufftComplex* spec = reinterpret_cast<cufftComplex*>(mesh);
     if (s->phi[m]) CUFFT_TRY(cufftExecR2C(s->r2c_d, s->phi[m], spec));
     else CUFFT_TRY(cufftExecR2C(s->r2c, mesh, spec));
-    const int nh = s->res / 2 + 1;
     if (s->zpass) {
-        launch_zpass(s, mesh, nh);
+        launch_zpass(s, mesh);
         CUFFT_TRY(cufftExecC2R(s->c2r_d, spec, s->phi[m]));
     } else {
         djb::k_kspace_mul<<<dim3(unsigned((s->res + djb::kSpecRows - 1) / djb::kSpecRows), unsigned(s->res)), kThreads,
@@ -1859,7 +1874,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             TRY(dmalloc(s, (void**)&s->phi[m], sizeof(float) * size_t(res) * res * res));
         {
             const char* zp = std::getenv("DJB_ZPASS");
-            s->zpass = (res == djb::kZRes) && !(zp && std::strcmp(zp, "0") == 0);
+            s->zpass = djb::zpass_size(res) && !(zp && std::strcmp(zp, "0") == 0);
         }
         // 3-D transforms, or with the fused z pass 2-D transforms batched over the z planes
         const int rank = s->zpass ? 2 : 3;
@@ -1889,14 +1904,10 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
                 w[j] = make_float2(float(std::cos(2 * M_PI * j / res)), float(-std::sin(2 * M_PI * j / res)));
             TRY(dmalloc(s, (void**)&s->wN, sizeof(float2) * res));
             CUDA_TRY(cudaMemcpy(s->wN, w.data(), sizeof(float2) * res, cudaMemcpyHostToDevice));
-            float2 w32[16];
-            for (int j = 0; j < 16; ++j)
-                w32[j] = make_float2(float(std::cos(2 * M_PI * j / 32)), float(-std::sin(2 * M_PI * j / 32)));
-            CUDA_TRY(cudaMemcpyToSymbol(djb::c_w32, w32, sizeof(w32)));
-            CUDA_TRY(cudaFuncSetAttribute(djb::k_zpencil_kphi<djb::KPhiFn>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, djb::kZSmem));
-            CUDA_TRY(cudaFuncSetAttribute(djb::k_zpencil_pair<djb::KPhiFn>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, djb::kZSmem));
+            if (res == 128) TRY(zpass_attrs<128>());
+            if (res == 256) TRY(zpass_attrs<256>());
+            if (res == 512) TRY(zpass_attrs<512>());
+            if (res == 1024) TRY(zpass_attrs<1024>());
         }
         const char* tm = std::getenv("DJB_TMA");   // DJB_TMA=0: boxes by asynchronous copies only
         if (s->sorted && s->gsx <= res && !(tm && std::strcmp(tm, "0") == 0)) {

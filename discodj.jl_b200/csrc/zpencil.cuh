@@ -1,5 +1,6 @@
-// Fused z pass of the Poisson solve on a 1024^3 mesh: forward DFT along z, the
-// multiplier Kφ, inverse DFT along z, in place on the half spectrum.
+// Fused z pass of the Poisson solve on meshes of 128, 256, 512 and 1024 cells per side:
+// forward DFT along z, the multiplier Kφ, inverse DFT along z, in place on the half
+// spectrum.
 //
 // The 3-D R2C / C2R transforms of the force calculation are split into a batched 2-D
 // transform of the z planes (cuFFT) and this kernel, which does both z transforms of
@@ -7,311 +8,215 @@
 // replaces three passes over the spectrum (the z stage of the forward transform, the
 // k-space multiplication and the z stage of the inverse transform) by one.
 //
-// Layout: spectrum f[(kz * res + ky) * nh + kx], nh = res/2 + 1 (the 2-D R2C halves x).
-// A CTA owns 8 consecutive kx of one ky: 8 pencils x 32 threads, thread (q, t) at
-// threadIdx.x = q + 8 t, so that a warp reads 4 kz rows of 8 consecutive kx (64 bytes
-// each) per load. res = 1024 = 32 x 32 (Cooley-Tukey with n = n2 + 32 n1 and
-// k = k1 + 32 k2):
-//   A  thread n2 loads x[n2 + 32 n1], DFT over n1 (radix-2 DIF in registers),
-//      multiplies by W^(n2 k1) (W = exp(-2 pi i / 1024)), writes to shared memory;
-//   B  thread k1 reads its row, DFT over n2 -> X[k1 + 32 k2]; X *= Kφ(kx, ky, kz);
-//   A' inverse DFT over k2 (radix-2 DIT on the bit-reversed registers), multiplies by
-//      W^-(n2 k1), writes back transposed;
-//   B' thread n2 reads its column, inverse DFT over k1 (DIF) -> x[n2 + 32 n1], stores.
-// Both transforms are unnormalised, as cuFFT's, so Kφ keeps its 1/res^3 factor.
-// Twiddles: W_32^j from a constant table (uniform across the warp), W^(n2 k1) from a
-// float table of the 1024 roots computed in float64 on the host.
+// Layout: spectrum f[(kz * N + ky) * nh + kx], nh = N/2 + 1 (the 2-D R2C halves x).
+// A CTA owns 16 consecutive kx of one ky: rows of 128 bytes. Rows of 64 bytes, half of
+// that, cost twice the time at N = 1024 (a plain read-modify-write of the spectrum in
+// this order: 1.5 ms with 128-byte rows, 2.9 ms with 64-byte rows): consecutive kz lie
+// 4 MB apart there, so each row is an address translation of its own.
+// N = 32 M (Cooley-Tukey with n = n2 + M n1 and k = k1 + 32 k2), 16 x M threads, thread
+// (q, t) at threadIdx.x = q + 16 t holding 32 points of pencil q in registers:
+//   A  loads x[t + M n1], DFT over n1 (radix-2 DIF), multiplies by W^(t k1)
+//      (W = exp(-2 pi i / N)), exchanges through shared memory;
+//   B  holds rows k1 = (32/M) t + j, DFT over n2 -> X[k1 + 32 k2]; X *= Kφ(kx, ky, kz);
+//   B' inverse DFT over k2 (radix-2 DIT on the bit-reversed registers), multiplies by
+//      W^-(n2 k1), exchanges back;
+//   A' inverse DFT over k1 (DIT) -> x[t + M n1], stored where A loaded.
+// Both transforms are unnormalised, as cuFFT's, so Kφ keeps its 1/N^3 factor. The
+// twiddles of the small DFTs are compile-time constants (multiplications by 1, -i and
+// the eighth roots cost nothing or two multiplications); W^(n2 k1) comes from a float
+// table of the N roots computed in float64 on the host.
+//
+// Measured (force phases of a step, per mesh): 1024^3 4.79 -> 4.19 ms against the earlier
+// form with 8 pencils per CTA on thread pairs; 512^3 0.85 + 0.24 + 0.86 ms (3-D transforms
+// and the multiplication) -> 0.53 + 0.45 + 0.54 ms. The arithmetic of the two DFTs and of
+// Kφ (about 100 lane instructions per mode) bounds it, not memory (1.5 ms at 1024^3).
 #pragma once
 
 #include <cstdint>
 
 namespace djb {
 
-#ifndef DJB_ZPASS_BLOCKS
-#define DJB_ZPASS_BLOCKS 2
-#endif
-#ifndef DJB_ZPASS_KTABLE
-#define DJB_ZPASS_KTABLE 0
-#endif
-
-constexpr int kZRes = 1024;
-#ifndef DJB_ZPASS_PENCILS
-#define DJB_ZPASS_PENCILS 8
-#endif
-constexpr int kZPencils = DJB_ZPASS_PENCILS;  // kx per CTA
-constexpr int kZThreads = kZPencils * 32;
-constexpr int kZRow = 33;              // shared row pitch (float2), breaks bank alignment
-constexpr int kZPlane = 32 * kZRow + 2;  // per-pencil block (float2)
-constexpr int kZKRow = kZRes + 4;        // Kφ row pitch (floats): the 8 pencils on different banks
-constexpr int kZSmem = kZPencils * kZPlane * 8 + (DJB_ZPASS_KTABLE ? kZPencils * kZKRow * 4 : 0);  // dynamic shared bytes
-
-__constant__ float2 c_w32[16];  // exp(-2 pi i j / 32), j < 16
+constexpr int kZPencils = 16;   // kx per CTA
+constexpr int kZPoints = 32;    // points per thread
+__host__ __device__ constexpr bool zpass_size(int res) { return res == 128 || res == 256 || res == 512 || res == 1024; }
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-
-__host__ __device__ constexpr int brev5(int i) {
-    return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
+__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {   // a conj(b)
+    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 
-// One radix-2 stage on blocks of LEN points (LEN a template constant, so every register
-// index below is a compile-time constant and the pencil stays in registers).
-template <int LEN>
-__device__ __forceinline__ void dif_stage(float2 (&a)[32]) {
-    constexpr int half = LEN / 2;
-#pragma unroll
-    for (int s = 0; s < 32; s += LEN) {
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            const float2 u = a[s + j], v = a[s + j + half];
-            a[s + j] = make_float2(u.x + v.x, u.y + v.y);
-            const float2 d = make_float2(u.x - v.x, u.y - v.y);
-            a[s + j + half] = (j == 0) ? d : cmul(d, c_w32[j * (32 / LEN)]);
-        }
+// cos(2 pi m / 32) for m = 0 .. 8
+__host__ __device__ constexpr float cos32(int m) {
+    return m == 0 ? 1.0f : m == 1 ? 0.98078528040323044913f : m == 2 ? 0.92387953251128675613f
+         : m == 3 ? 0.83146961230254523708f : m == 4 ? 0.70710678118654752440f : m == 5 ? 0.55557023301960222474f
+         : m == 6 ? 0.38268343236508977173f : m == 7 ? 0.19509032201612826785f : 0.0f;
+}
+
+// d exp(-+2 pi i m / 32) for 0 <= m < 16, m a constant after unrolling (INV: + sign).
+template <bool INV>
+__device__ __forceinline__ float2 twiddle32(float2 d, int m) {
+    if (m == 0) return d;
+    if (m == 8) return INV ? make_float2(-d.y, d.x) : make_float2(d.y, -d.x);
+    if (m == 4) {
+        constexpr float c = cos32(4);
+        return INV ? make_float2((d.x - d.y) * c, (d.x + d.y) * c) : make_float2((d.x + d.y) * c, (d.y - d.x) * c);
     }
+    if (m == 12) {
+        constexpr float c = cos32(4);
+        return INV ? make_float2((d.x + d.y) * -c, (d.x - d.y) * c) : make_float2((d.y - d.x) * c, (d.x + d.y) * -c);
+    }
+    const float wr = m < 8 ? cos32(m) : -cos32(16 - m);
+    const float wi = m < 8 ? cos32(8 - m) : cos32(m - 8);   // sin(2 pi m / 32)
+    return INV ? make_float2(d.x * wr - d.y * wi, d.y * wr + d.x * wi)
+               : make_float2(d.x * wr + d.y * wi, d.y * wr - d.x * wi);
 }
 
-template <int LEN>
-__device__ __forceinline__ void dit_stage(float2 (&a)[32]) {
-    constexpr int half = LEN / 2;
+// L-point DFTs on consecutive groups of L of the 32 registers. DIF: natural order in,
+// bit-reversed out; DIT: bit-reversed in, natural out.
+template <int LEN, bool INV>
+__device__ __forceinline__ void dif_stage(float2 (&a)[kZPoints]) {
 #pragma unroll
-    for (int s = 0; s < 32; s += LEN) {
+    for (int s = 0; s < kZPoints; s += LEN)
 #pragma unroll
-        for (int j = 0; j < half; ++j) {
+        for (int j = 0; j < LEN / 2; ++j) {
+            const float2 u = a[s + j], v = a[s + j + LEN / 2];
+            a[s + j] = make_float2(u.x + v.x, u.y + v.y);
+            a[s + j + LEN / 2] = twiddle32<INV>(make_float2(u.x - v.x, u.y - v.y), j * (32 / LEN));
+        }
+}
+template <int LEN, bool INV>
+__device__ __forceinline__ void dit_stage(float2 (&a)[kZPoints]) {
+#pragma unroll
+    for (int s = 0; s < kZPoints; s += LEN)
+#pragma unroll
+        for (int j = 0; j < LEN / 2; ++j) {
             const float2 u = a[s + j];
-            const float2 v = (j == 0) ? a[s + j + half] : cmul(a[s + j + half], c_w32[j * (32 / LEN)]);
+            const float2 v = twiddle32<INV>(a[s + j + LEN / 2], j * (32 / LEN));
             a[s + j] = make_float2(u.x + v.x, u.y + v.y);
-            a[s + j + half] = make_float2(u.x - v.x, u.y - v.y);
+            a[s + j + LEN / 2] = make_float2(u.x - v.x, u.y - v.y);
         }
+}
+template <int L, bool INV>
+__device__ __forceinline__ void dft_dif(float2 (&a)[kZPoints]) {
+    if constexpr (L >= 32) dif_stage<32, INV>(a);
+    if constexpr (L >= 16) dif_stage<16, INV>(a);
+    if constexpr (L >= 8) dif_stage<8, INV>(a);
+    if constexpr (L >= 4) dif_stage<4, INV>(a);
+    dif_stage<2, INV>(a);
+}
+template <int L, bool INV>
+__device__ __forceinline__ void dft_dit(float2 (&a)[kZPoints]) {
+    dit_stage<2, INV>(a);
+    if constexpr (L >= 4) dit_stage<4, INV>(a);
+    if constexpr (L >= 8) dit_stage<8, INV>(a);
+    if constexpr (L >= 16) dit_stage<16, INV>(a);
+    if constexpr (L >= 32) dit_stage<32, INV>(a);
+}
+
+// Bit reversal of i < L (L a power of two).
+template <int L>
+__host__ __device__ constexpr int brev(int i) {
+    int r = 0;
+    for (int b = 1; b < L; b <<= 1) r = 2 * r + ((i & b) ? 1 : 0);
+    return r;
+}
+
+// Shared memory: the N twiddles, then the exchange area [k1][n2][pencil], rows of k1
+// padded so that the two threads t of a warp read from different banks: float2 elements,
+// or at N = 1024 one component at a time (float elements), which leaves two CTAs' worth
+// of shared memory to the L1 cache.
+template <int N>
+struct ZGeom {
+    static constexpr int M = N / kZPoints;              // threads per pencil
+    static constexpr int kThreads = kZPencils * M;
+    static constexpr int J = 32 / M;                    // rows per thread in stage B
+    static constexpr bool kSplit = N == 1024;           // exchange one component at a time
+    static constexpr int kPad = kSplit ? 16 : 0;        // J * row = 16 modulo 32 words
+    static constexpr int kRow = M * kZPencils + kPad;   // elements per k1
+    static constexpr size_t kSmem = size_t(N) * 8 + size_t(32) * kRow * (kSplit ? 4 : 8);
+    static constexpr int kBlocks = N == 1024 ? 1 : (N == 512 ? 2 : (N == 256 ? 4 : 8));   // 128 registers per thread
+};
+
+// Registers a[R(c)] of stage A (c = k1) against stage B's rows through the exchange area.
+// to_rows: thread (q, t) writes a[brev(k1)] at (k1, n2 = t) and reads (k1 = J t + j, n2)
+// into a[j M + n2]; otherwise the reverse, into a[brev(k1)]. A thread starts the second
+// exchange by writing the slots that it alone read last in the first: no barrier between.
+template <int N, bool TO_ROWS>
+__device__ __forceinline__ void zexchange(float2 (&a)[kZPoints], void* area, int q, int t) {
+    using G = ZGeom<N>;
+    constexpr int M = G::M, J = G::J;
+    const int ca = t * kZPencils + q;          // + k1 * row
+    const int cb = J * t * G::kRow + q;        // + j * row + n2 * 16
+    if constexpr (G::kSplit) {
+        float* e = static_cast<float*>(area);
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+            if (part) __syncthreads();   // the first component has been read
+#pragma unroll
+            for (int i = 0; i < kZPoints; ++i) {
+                const int at = TO_ROWS ? ca + brev<32>(i) * G::kRow : cb + (i / M) * G::kRow + (i % M) * kZPencils;
+                e[at] = part ? a[i].y : a[i].x;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < kZPoints; ++i) {
+                const int at = TO_ROWS ? cb + (i / M) * G::kRow + (i % M) * kZPencils : ca + brev<32>(i) * G::kRow;
+                (part ? a[i].y : a[i].x) = e[at];
+            }
+        }
+    } else {
+        float2* e = static_cast<float2*>(area);
+#pragma unroll
+        for (int i = 0; i < kZPoints; ++i)
+            e[TO_ROWS ? ca + brev<32>(i) * G::kRow : cb + (i / M) * G::kRow + (i % M) * kZPencils] = a[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kZPoints; ++i)
+            a[i] = e[TO_ROWS ? cb + (i / M) * G::kRow + (i % M) * kZPencils : ca + brev<32>(i) * G::kRow];
     }
 }
 
-// Radix-2 decimation in frequency, natural order in, bit-reversed order out (forward).
-__device__ __forceinline__ void dft32_dif(float2 (&a)[32]) {
-    dif_stage<32>(a);
-    dif_stage<16>(a);
-    dif_stage<8>(a);
-    dif_stage<4>(a);
-    dif_stage<2>(a);
-}
-
-// Radix-2 decimation in time, bit-reversed order in, natural order out (forward).
-__device__ __forceinline__ void dft32_dit(float2 (&a)[32]) {
-    dit_stage<2>(a);
-    dit_stage<4>(a);
-    dit_stage<8>(a);
-    dit_stage<16>(a);
-    dit_stage<32>(a);
-}
-
-// kphi(kx, ky, kz): the multiplier. One CTA per (ky, 8 kx) tile. By default Kφ is
-// evaluated in step B with float64 sums and products and one float division
-// (KPhiFn::fast, within 1.5 ulp of the float64 quotient); DJB_ZPASS_KTABLE = 1 evaluates
-// the float64 quotient for the tile into shared memory before the pencils are loaded
-// (measured 9% slower on the 1024^3 step).
-template <class KPhi>
-__global__ void __launch_bounds__(kZThreads, DJB_ZPASS_BLOCKS) k_zpencil_kphi(float2* __restrict__ f, int nh,
-                                                                             const float2* __restrict__ wN,
-                                                                             KPhi kphi) {
-    extern __shared__ __align__(16) float2 s[];  // kZPencils transpose blocks (then Kφ rows)
-    const int q = threadIdx.x & (kZPencils - 1);
-    const int t = threadIdx.x / kZPencils;  // n2 (steps A, B'), k1 (steps B, A')
-    const int ky = blockIdx.y;
-    const int kx = blockIdx.x * kZPencils + q;
+template <int N, class KPhi>
+__global__ void __launch_bounds__(ZGeom<N>::kThreads, ZGeom<N>::kBlocks) k_zpass(
+    float2* __restrict__ f, const float2* __restrict__ wN, KPhi kphi) {
+    using G = ZGeom<N>;
+    constexpr int M = G::M, J = G::J, nh = N / 2 + 1;
+    extern __shared__ __align__(16) unsigned char zs[];
+    float2* const w = reinterpret_cast<float2*>(zs);
+    void* const area = zs + size_t(N) * 8;
+    const int q = threadIdx.x % kZPencils, t = threadIdx.x / kZPencils;
+    const int ky = blockIdx.y, kx = blockIdx.x * kZPencils + q;
     const bool active = kx < nh;
-#if DJB_ZPASS_KTABLE
-    float* const sK = reinterpret_cast<float*>(s + kZPencils * kZPlane);
-    for (int e = threadIdx.x; e < kZPencils * kZRes; e += kZThreads) {
-        const int qq = e / kZRes, kz = e - qq * kZRes;
-        const int kxx = blockIdx.x * kZPencils + qq;
-        sK[qq * kZKRow + kz] = (kxx < nh) ? kphi(kxx, ky, kz) : 0.0f;
-    }
-#endif
-    const int64_t zstride = int64_t(kZRes) * nh;
-    float2* __restrict__ col = f + int64_t(ky) * nh + (active ? kx : 0);
-    float2* const sq = s + q * kZPlane;
-    float2 a[32];
-    // A: x[t + 32 n1], n1 = 0..31
+    constexpr int64_t zstride = int64_t(N) * nh;
+    float2* __restrict__ const col = f + int64_t(ky) * nh + (active ? kx : 0) + t * zstride;
+    float2 a[kZPoints];
 #pragma unroll
-    for (int n1 = 0; n1 < 32; ++n1)
-        a[n1] = active ? __ldcs(col + int64_t(t + 32 * n1) * zstride) : make_float2(0.f, 0.f);
-    dft32_dif(a);  // a[i] = Y[k1 = brev(i)]
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        const int k1 = brev5(i);
-        sq[k1 * kZRow + t] = (k1 == 0) ? a[i] : cmul(a[i], __ldg(wN + ((t * k1) & (kZRes - 1))));
-    }
-    __syncthreads();  // transpose block (and Kφ rows) complete
-    // B: thread k1 = t: DFT over n2
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) a[n2] = sq[t * kZRow + n2];
-    dft32_dif(a);  // a[i] = X[t + 32 brev(i)]
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-#if DJB_ZPASS_KTABLE
-        const float K = sK[q * kZKRow + t + 32 * brev5(i)];
-#else
-        const float K = kphi.fast(kx, ky, t + 32 * brev5(i));
-#endif
-        a[i] = make_float2(a[i].x * K, -(a[i].y * K));  // conjugated for the inverse below
-    }
-    // A': inverse DFT over k2 (input bit-reversed) -> Z[k1 = t][n2], n2 natural; row t of
-    // the transpose block is read and written by this thread only
-    dft32_dit(a);
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2) {
-        const float2 z = conjf2(a[n2]);
-        sq[t * kZRow + n2] = (t == 0 || n2 == 0) ? z : cmul(z, conjf2(__ldg(wN + ((n2 * t) & (kZRes - 1)))));
-    }
+    for (int i = 0; i < kZPoints; ++i)
+        a[i] = active ? __ldcs(col + int64_t(M * i) * zstride) : make_float2(0.0f, 0.0f);
+    for (int i = threadIdx.x; i < N; i += G::kThreads) w[i] = wN[i];
     __syncthreads();
-    // B': thread n2 = t: inverse DFT over k1 -> x[t + 32 n1]
+    dft_dif<32, false>(a);   // a[i] = Y[k1 = brev(i)] of n2 = t
 #pragma unroll
-    for (int k1 = 0; k1 < 32; ++k1) a[k1] = conjf2(sq[k1 * kZRow + t]);
-    dft32_dif(a);  // a[i] = conj(x[t + 32 brev(i)])
+    for (int i = 1; i < kZPoints; ++i) a[i] = cmul(a[i], w[(t * brev<32>(i)) & (N - 1)]);
+    zexchange<N, true>(a, area, q, t);
+    dft_dif<M, false>(a);    // a[j M + i] = X[k1 + 32 brev(i)], k1 = J t + j
+    const typename KPhi::Pencil kp = kphi.pencil(active ? kx : 0, ky);
+#pragma unroll
+    for (int i = 0; i < kZPoints; ++i) {
+        const float K = kphi.at(kp, J * t + i / M + 32 * brev<M>(i % M));
+        a[i] = make_float2(a[i].x * K, a[i].y * K);
+    }
+    dft_dit<M, true>(a);     // a[j M + n2]
+#pragma unroll
+    for (int i = 0; i < kZPoints; ++i)
+        if (i % M != 0) a[i] = cmulc(a[i], w[((i % M) * (J * t + i / M)) & (N - 1)]);
+    zexchange<N, false>(a, area, q, t);
+    dft_dit<32, true>(a);    // a[i] = x[t + M i]
     if (active) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) __stcs(col + int64_t(t + 32 * brev5(i)) * zstride, conjf2(a[i]));
-    }
-}
-
-// ── pencil transforms on thread pairs ───────────────────────────────────────
-// The same transform with each 32-point DFT split over two threads (lanes 8 apart):
-// thread h of the pair holds points 16h .. 16h + 15. The radix-2 stage of length 32
-// pairs point j with j + 16, i.e. the two threads, and exchanges them with one
-// shuffle per point; the stages of length 16 .. 2 stay inside each thread. Half the
-// registers per thread (16 points) let twice as many warps share an SM, which the pass
-// needs to keep enough loads in flight (it is bound by load latency).
-#ifndef DJB_ZPASS_PAIR
-#define DJB_ZPASS_PAIR 1
-#endif
-constexpr int kZPairThreads = kZPencils * 64;
-
-template <int LEN>
-__device__ __forceinline__ void dif_stage16(float2 (&b)[16]) {
-    constexpr int half = LEN / 2;
-#pragma unroll
-    for (int s = 0; s < 16; s += LEN) {
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            const float2 u = b[s + j], v = b[s + j + half];
-            b[s + j] = make_float2(u.x + v.x, u.y + v.y);
-            const float2 d = make_float2(u.x - v.x, u.y - v.y);
-            b[s + j + half] = (j == 0) ? d : cmul(d, c_w32[j * (32 / LEN)]);
-        }
-    }
-}
-
-template <int LEN>
-__device__ __forceinline__ void dit_stage16(float2 (&b)[16]) {
-    constexpr int half = LEN / 2;
-#pragma unroll
-    for (int s = 0; s < 16; s += LEN) {
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            const float2 u = b[s + j];
-            const float2 v = (j == 0) ? b[s + j + half] : cmul(b[s + j + half], c_w32[j * (32 / LEN)]);
-            b[s + j] = make_float2(u.x + v.x, u.y + v.y);
-            b[s + j + half] = make_float2(u.x - v.x, u.y - v.y);
-        }
-    }
-}
-
-// The partner of the pair is `P` lanes away (P pencils per CTA, P = 8 or 16).
-template <int P>
-__device__ __forceinline__ float2 shfl_pair(float2 v) {
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, P), __shfl_xor_sync(0xffffffffu, v.y, P));
-}
-
-// Forward DIF over the pair: natural order in, bit-reversed order out (position 16h + i).
-template <int P>
-__device__ __forceinline__ void dft32_dif_pair(float2 (&b)[16], int h) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float2 o = shfl_pair<P>(b[j]);
-        if (h == 0) {
-            b[j] = make_float2(b[j].x + o.x, b[j].y + o.y);
-        } else {
-            const float2 d = make_float2(o.x - b[j].x, o.y - b[j].y);
-            b[j] = (j == 0) ? d : cmul(d, c_w32[j]);
-        }
-    }
-    dif_stage16<16>(b);
-    dif_stage16<8>(b);
-    dif_stage16<4>(b);
-    dif_stage16<2>(b);
-}
-
-// Forward DIT over the pair: bit-reversed order in, natural order out.
-template <int P>
-__device__ __forceinline__ void dft32_dit_pair(float2 (&b)[16], int h) {
-    dit_stage16<2>(b);
-    dit_stage16<4>(b);
-    dit_stage16<8>(b);
-    dit_stage16<16>(b);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float2 m = (h == 1 && j > 0) ? cmul(b[j], c_w32[j]) : b[j];
-        const float2 o = shfl_pair<P>(m);
-        b[j] = (h == 0) ? make_float2(m.x + o.x, m.y + o.y) : make_float2(o.x - m.x, o.y - m.y);
-    }
-}
-
-// P pencils per CTA of 64·P threads. Thread (q, h, t) at threadIdx.x = q + P h + 2P t:
-// pencil q, half h, and t = n2 (steps A, B') or k1 (steps B, A'); a warp reads 32/P kz
-// row pairs of P consecutive kx (8·P bytes each) per load.
-template <class KPhi, int P = 8>
-__global__ void __launch_bounds__(64 * P, P == 8 ? 2 : 1) k_zpencil_pair(float2* __restrict__ f, int nh,
-                                                                         const float2* __restrict__ wN, KPhi kphi) {
-    extern __shared__ __align__(16) float2 s[];  // P transpose blocks
-    const int q = threadIdx.x & (P - 1);
-    const int h = (threadIdx.x / P) & 1;
-    const int t = threadIdx.x / (2 * P);
-    const int ky = blockIdx.y;
-    const int kx = blockIdx.x * P + q;
-    const bool active = kx < nh;
-    const int64_t zstride = int64_t(kZRes) * nh;
-    float2* __restrict__ col = f + int64_t(ky) * nh + (active ? kx : 0);
-    float2* const sq = s + q * kZPlane;
-    float2 b[16];
-    // A: x[t + 32 n1], n1 = 16 h + i
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-        b[i] = active ? __ldcs(col + int64_t(t + 32 * (16 * h + i)) * zstride) : make_float2(0.f, 0.f);
-    dft32_dif_pair<P>(b, h);  // b[i] = Y[k1 = brev(16h + i)]
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int k1 = brev5(16 * h + i);
-        sq[k1 * kZRow + t] = (k1 == 0) ? b[i] : cmul(b[i], __ldg(wN + ((t * k1) & (kZRes - 1))));
-    }
-    __syncthreads();
-    // B: thread pair k1 = t: DFT over n2 (this thread: n2 = 16 h + i)
-#pragma unroll
-    for (int i = 0; i < 16; ++i) b[i] = sq[t * kZRow + 16 * h + i];
-    dft32_dif_pair<P>(b, h);  // b[i] = X[t + 32 brev(16h + i)]
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float K = kphi.fast(kx, ky, t + 32 * brev5(16 * h + i));
-        b[i] = make_float2(b[i].x * K, -(b[i].y * K));  // conjugated for the inverse below
-    }
-    // A': inverse DFT over k2 -> Z[k1 = t][n2 = 16 h + i]; this thread reads and writes
-    // only its half of row t
-    dft32_dit_pair<P>(b, h);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int n2 = 16 * h + i;
-        const float2 z = conjf2(b[i]);
-        sq[t * kZRow + n2] = (t == 0 || n2 == 0) ? z : cmul(z, conjf2(__ldg(wN + ((n2 * t) & (kZRes - 1)))));
-    }
-    __syncthreads();
-    // B': thread pair n2 = t: inverse DFT over k1 (this thread: k1 = 16 h + i)
-#pragma unroll
-    for (int i = 0; i < 16; ++i) b[i] = conjf2(sq[(16 * h + i) * kZRow + t]);
-    dft32_dif_pair<P>(b, h);  // b[i] = conj(x[t + 32 brev(16h + i)])
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) __stcs(col + int64_t(t + 32 * brev5(16 * h + i)) * zstride, conjf2(b[i]));
+        for (int i = 0; i < kZPoints; ++i) __stcs(col + int64_t(M * i) * zstride, a[i]);
     }
 }
 

@@ -266,3 +266,23 @@ def test_fused_z_pass_matches_3d_transforms(djb, monkeypatch):
     with djb.PMSolver(cfg) as B:
         b = B.acceleration(psi)
     assert rel(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("res,n,W,lap,dec", [(128, 50, 4, 0, True), (256, 64, 3, 4, False), (512, 48, 2, 0, False),
+                                             (512, 70, 4, 6, True)])
+def test_fused_z_pass_sizes_match_3d_transforms(djb, monkeypatch, res, n, W, lap, dec):
+    """The fused z pass at its smaller sizes (one kernel instance each; the last group of 16
+    kx holds one pencil) against the 3-D transforms with the separate multiplication. Both
+    are float32 transforms of the same density: a few 1e-7 per transform, amplified by the
+    deconvolution; 1e-5 as at 1024^3."""
+    rng = np.random.default_rng(res + n)
+    L = 100.0
+    psi = (5 * rng.standard_normal((n, n, n, 3))).astype(np.float32)
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=L, worder=W, antialias=1, grad_order=4, lap_order=lap,
+                       deconvolve=dec)
+    with djb.PMSolver(cfg) as A:
+        a = A.acceleration(psi)
+    monkeypatch.setenv("DJB_ZPASS", "0")
+    with djb.PMSolver(cfg) as B:
+        b = B.acceleration(psi)
+    assert rel(a, b) < 1e-5
