@@ -729,24 +729,33 @@ __global__ void k_wrap_psi_lin(const float* __restrict__ psi, const float* __res
 #include "adjoint.cuh"
 
 namespace djb {
-// Kφ as a functor for the fused z pass: float64 sums and products, one float division
-// (within 1.5 ulp of kphi).
+// Kφ as a functor for the fused z pass: float64 sums and products; the quotient in
+// float32 from an approximate reciprocal and one step on its residual (within 1.5 ulp of
+// kphi). The table of the inverse Laplacian and the numerator carry a common power of two
+// (`scale`) that brings (2 pi / L)^2 to 1 .. 4, so no divisor is subnormal in any unit of length.
 struct KPhiFn {
     const double* T;
     const double* M;
-    double s0;
+    double s0;      // times scale
+    double scale;
     struct Pencil {
         double t, num;
         float numf;
         bool dc;
     };
-    __device__ __forceinline__ Pencil pencil(int kx, int ky) const {
-        const double num = M ? s0 * (M[kx] * M[ky]) : s0;
-        return Pencil{T[kx] + T[ky], num, float(num), (kx | ky) == 0};
+    // t, m: the tables T * scale and M in shared memory
+    __device__ __forceinline__ Pencil pencil(int kx, int ky, const double* t, const double* m) const {
+        const double num = M ? s0 * (m[kx] * m[ky]) : s0;
+        return Pencil{t[kx] + t[ky], num, float(num), (kx | ky) == 0};
     }
-    __device__ __forceinline__ float at(const Pencil& p, int kz) const {
-        if (p.dc && kz == 0) return 0.0f;
-        return (M ? float(p.num * __ldg(M + kz)) : p.numf) / float(p.t + __ldg(T + kz));
+    __device__ __forceinline__ float at(const Pencil& p, int kz, const double* t, const double* m) const {
+        const float num = M ? float(p.num * m[kz]) : p.numf;
+        const float den = float(p.t + t[kz]);
+        float r;
+        asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(den));
+        const float k = num * r;
+        const float v = fmaf(fmaf(-den, k, num), r, k);
+        return (p.dc && kz == 0) ? 0.0f : v;
     }
 };
 }  // namespace djb
@@ -837,6 +846,7 @@ struct djb_solver {
     std::vector<double> rshifts;    // resampling offsets, 3 per offset
     float c1 = 0, c2 = 0, c3 = 0;   // FD coefficients (pm.jl:419-424)
     double s0 = 0;                  // Kφ scale
+    double kscale = 1;              // power of two that brings (2π/L)² to 1 .. 4 (fused z pass)
 
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
@@ -1303,9 +1313,10 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
 template <int N>
 void launch_zpass_n(djb_solver* s, float* mesh) {
     using G = djb::ZGeom<N>;
-    const dim3 grid(unsigned((N / 2 + djb::kZPencils) / djb::kZPencils), unsigned(N));
-    djb::k_zpass<N><<<grid, G::kThreads, G::kSmem, s->stream>>>(reinterpret_cast<float2*>(mesh), s->wN,
-                                                                djb::KPhiFn{s->lapT, s->makT, s->s0});
+    const int tiles = N * (N / 2 + 1) / djb::kZPencils;
+    djb::k_zpass<N><<<std::min(tiles, s->nsm * G::kBlocks), G::kThreads, G::kSmem, s->stream>>>(reinterpret_cast<float2*>(mesh), s->wN,
+                                                                djb::KPhiFn{s->lapT, s->makT, s->s0 * s->kscale,
+                                                                            s->kscale});
 }
 
 void launch_zpass(djb_solver* s, float* mesh) {
@@ -1319,6 +1330,8 @@ template <int N>
 int zpass_attrs() {
     CUDA_TRY(cudaFuncSetAttribute(djb::k_zpass<N, djb::KPhiFn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(djb::ZGeom<N>::kSmem)));
+    CUDA_TRY(cudaFuncSetAttribute(djb::k_zpass<N, djb::KPhiFn>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  int(cudaSharedmemCarveoutMaxShared)));
     return DJB_OK;
 }
 
@@ -1781,6 +1794,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
     const int res = s->res;
     std::vector<double> T(res), M(res);
     const double dk = 2 * M_PI / s->L;
+    if (dk * dk > 0.0 && std::isfinite(dk * dk)) s->kscale = std::ldexp(1.0, -std::ilogb(dk * dk));
     const double mm = (res / 2) * dk / M_PI;  // maximum(abs.(k))/π = res/L
     for (int i = 0; i < res; ++i) {
         const double k = (i < res / 2 ? i : i - res) * 2 * M_PI / s->L;

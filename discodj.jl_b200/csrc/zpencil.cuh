@@ -8,11 +8,16 @@
 // replaces three passes over the spectrum (the z stage of the forward transform, the
 // k-space multiplication and the z stage of the inverse transform) by one.
 //
-// Layout: spectrum f[(kz * N + ky) * nh + kx], nh = N/2 + 1 (the 2-D R2C halves x).
-// A CTA owns 16 consecutive kx of one ky: rows of 128 bytes. Rows of 64 bytes, half of
-// that, cost twice the time at N = 1024 (a plain read-modify-write of the spectrum in
-// this order: 1.5 ms with 128-byte rows, 2.9 ms with 64-byte rows): consecutive kz lie
-// 4 MB apart there, so each row is an address translation of its own.
+// Layout: spectrum f[kz][pencil], pencil = ky * nh + kx, nh = N/2 + 1 (the 2-D R2C halves
+// x). A tile is 16 consecutive pencils of this flat plane: per kz one 128-byte line (the
+// plane is a multiple of 16 pencils, so no line is split and no tile is partly empty).
+// Lines of 64 bytes cost twice the time at N = 1024 (a plain read-modify-write of the
+// spectrum in this order: 1.5 ms with 128-byte lines, 2.9 ms with 64): consecutive kz lie
+// 4 MB apart there, so each line is an address translation of its own. A persistent CTA
+// takes every gridDim-th tile; each thread copies its own points of the next tile to its
+// private slots in shared memory (8-byte asynchronous copies, no barrier) while it
+// transforms this one, which is what hides the load latency: with loads straight to
+// registers the warps waited for them three quarters of the time (issue slots 42% used).
 // N = 32 M (Cooley-Tukey with n = n2 + M n1 and k = k1 + 32 k2), 16 x M threads, thread
 // (q, t) at threadIdx.x = q + 16 t holding 32 points of pencil q in registers:
 //   A  loads x[t + M n1], DFT over n1 (radix-2 DIF), multiplies by W^(t k1)
@@ -26,17 +31,19 @@
 // the eighth roots cost nothing or two multiplications); W^(n2 k1) comes from a float
 // table of the N roots computed in float64 on the host.
 //
-// Measured (force phases of a step, per mesh): 1024^3 4.79 -> 4.19 ms against the earlier
-// form with 8 pencils per CTA on thread pairs; 512^3 0.85 + 0.24 + 0.86 ms (3-D transforms
-// and the multiplication) -> 0.53 + 0.45 + 0.54 ms. The arithmetic of the two DFTs and of
-// Kφ (about 100 lane instructions per mode) bounds it, not memory (1.5 ms at 1024^3).
+// Measured per mesh: 1024^3 4.79 ms (8 pencils per CTA on thread pairs) -> 4.19 (this split,
+// loads to registers) -> 3.44 (prefetch) -> 3.24 (twiddles at constant distances, one
+// reciprocal per mode); 512^3 0.45 -> 0.40 -> 0.37 ms, where the 3-D transforms with the
+// multiplication took 0.85 + 0.24 + 0.86 ms and the 2-D ones take 0.53 + 0.54. About 85
+// instructions per mode for 16 bytes moved: the issue slots are half busy (four warps per
+// scheduler, all that 128 registers allow), memory would allow 1.5 ms at 1024^3.
 #pragma once
 
 #include <cstdint>
 
 namespace djb {
 
-constexpr int kZPencils = 16;   // kx per CTA
+constexpr int kZPencils = 16;   // pencils per tile
 constexpr int kZPoints = 32;    // points per thread
 __host__ __device__ constexpr bool zpass_size(int res) { return res == 128 || res == 256 || res == 512 || res == 1024; }
 
@@ -123,58 +130,48 @@ __host__ __device__ constexpr int brev(int i) {
     return r;
 }
 
-// Shared memory: the N twiddles, then the exchange area [k1][n2][pencil], rows of k1
-// padded so that the two threads t of a warp read from different banks: float2 elements,
-// or at N = 1024 one component at a time (float elements), which leaves two CTAs' worth
-// of shared memory to the L1 cache.
+// Shared memory: the tables (the N twiddles W^(k1 n2) at k1 M + n2, so that every thread
+// reads its own at constant distances from one base; N terms of the inverse Laplacian, with
+// deconvolution N window factors), the prefetch slots [n1][thread], and the exchange area
+// [k1][n2][pencil] of one float per point (real and imaginary parts are exchanged one
+// after the other), rows of k1 padded so that the two threads t of a warp read different
+// banks. 128 registers per thread and about 200 KB of shared memory per SM.
 template <int N>
 struct ZGeom {
     static constexpr int M = N / kZPoints;              // threads per pencil
     static constexpr int kThreads = kZPencils * M;
     static constexpr int J = 32 / M;                    // rows per thread in stage B
-    static constexpr bool kSplit = N == 1024;           // exchange one component at a time
-    static constexpr int kPad = kSplit ? 16 : 0;        // J * row = 16 modulo 32 words
-    static constexpr int kRow = M * kZPencils + kPad;   // elements per k1
-    static constexpr size_t kSmem = size_t(N) * 8 + size_t(32) * kRow * (kSplit ? 4 : 8);
-    static constexpr int kBlocks = N == 1024 ? 1 : (N == 512 ? 2 : (N == 256 ? 4 : 8));   // 128 registers per thread
+    static constexpr int kRow = M * kZPencils + 16 / J; // words per k1: J rows = 16 modulo 32
+    static constexpr size_t kStage = size_t(kZPoints) * kThreads * 8;
+    static constexpr size_t kSmem = size_t(N) * 24 + kStage + size_t(32) * kRow * 4;
+    static constexpr int kBlocks = 1024 / N;            // CTAs per SM
 };
 
-// Registers a[R(c)] of stage A (c = k1) against stage B's rows through the exchange area.
-// to_rows: thread (q, t) writes a[brev(k1)] at (k1, n2 = t) and reads (k1 = J t + j, n2)
-// into a[j M + n2]; otherwise the reverse, into a[brev(k1)]. A thread starts the second
-// exchange by writing the slots that it alone read last in the first: no barrier between.
+// Registers of stage A (a[i] = point k1 = brev(i) of column n2 = t) to stage B's rows
+// (a[j M + n2], k1 = J t + j) or back. A thread starts an exchange by writing the slots that
+// it alone read at the end of the one before, so no barrier stands between exchanges.
 template <int N, bool TO_ROWS>
-__device__ __forceinline__ void zexchange(float2 (&a)[kZPoints], void* area, int q, int t) {
+__device__ __forceinline__ void zexchange(float2 (&a)[kZPoints], float* e, int q, int t) {
     using G = ZGeom<N>;
-    constexpr int M = G::M, J = G::J;
-    const int ca = t * kZPencils + q;          // + k1 * row
-    const int cb = J * t * G::kRow + q;        // + j * row + n2 * 16
-    if constexpr (G::kSplit) {
-        float* e = static_cast<float*>(area);
+    constexpr int M = G::M;
+    float* const ca = e + t * kZPencils + q;               // + k1 * row
+    float* const cb = e + G::J * t * G::kRow + q;          // + j * row + n2 * 16
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {
-            if (part) __syncthreads();   // the first component has been read
+    for (int part = 0; part < 2; ++part) {
+        if (part) __syncthreads();   // the first component has been read
 #pragma unroll
-            for (int i = 0; i < kZPoints; ++i) {
-                const int at = TO_ROWS ? ca + brev<32>(i) * G::kRow : cb + (i / M) * G::kRow + (i % M) * kZPencils;
-                e[at] = part ? a[i].y : a[i].x;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < kZPoints; ++i) {
-                const int at = TO_ROWS ? cb + (i / M) * G::kRow + (i % M) * kZPencils : ca + brev<32>(i) * G::kRow;
-                (part ? a[i].y : a[i].x) = e[at];
-            }
+        for (int i = 0; i < kZPoints; ++i) {
+            const float v = part ? a[i].y : a[i].x;
+            if (TO_ROWS) ca[brev<32>(i) * G::kRow] = v;
+            else cb[(i / M) * G::kRow + (i % M) * kZPencils] = v;
         }
-    } else {
-        float2* e = static_cast<float2*>(area);
-#pragma unroll
-        for (int i = 0; i < kZPoints; ++i)
-            e[TO_ROWS ? ca + brev<32>(i) * G::kRow : cb + (i / M) * G::kRow + (i % M) * kZPencils] = a[i];
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < kZPoints; ++i)
-            a[i] = e[TO_ROWS ? cb + (i / M) * G::kRow + (i % M) * kZPencils : ca + brev<32>(i) * G::kRow];
+        for (int i = 0; i < kZPoints; ++i) {
+            const float v = TO_ROWS ? cb[(i / M) * G::kRow + (i % M) * kZPencils] : ca[brev<32>(i) * G::kRow];
+            if (part) a[i].y = v;
+            else a[i].x = v;
+        }
     }
 }
 
@@ -183,41 +180,63 @@ __global__ void __launch_bounds__(ZGeom<N>::kThreads, ZGeom<N>::kBlocks) k_zpass
     float2* __restrict__ f, const float2* __restrict__ wN, KPhi kphi) {
     using G = ZGeom<N>;
     constexpr int M = G::M, J = G::J, nh = N / 2 + 1;
+    constexpr int64_t plane = int64_t(N) * nh;
+    constexpr int kTiles = int(plane / kZPencils);
     extern __shared__ __align__(16) unsigned char zs[];
     float2* const w = reinterpret_cast<float2*>(zs);
-    void* const area = zs + size_t(N) * 8;
+    double* const T = reinterpret_cast<double*>(zs + size_t(N) * 8);
+    double* const D = T + N;
+    float2* const stage = reinterpret_cast<float2*>(zs + size_t(N) * 24) + threadIdx.x;
+    float* const area = reinterpret_cast<float*>(zs + size_t(N) * 24 + G::kStage);
     const int q = threadIdx.x % kZPencils, t = threadIdx.x / kZPencils;
-    const int ky = blockIdx.y, kx = blockIdx.x * kZPencils + q;
-    const bool active = kx < nh;
-    constexpr int64_t zstride = int64_t(N) * nh;
-    float2* __restrict__ const col = f + int64_t(ky) * nh + (active ? kx : 0) + t * zstride;
-    float2 a[kZPoints];
+    const auto fetch = [&](int tile) {   // this thread's points of the tile to its slots
+        if (tile < kTiles) {
+            const float2* src = f + int64_t(tile) * kZPencils + q + t * plane;
 #pragma unroll
-    for (int i = 0; i < kZPoints; ++i)
-        a[i] = active ? __ldcs(col + int64_t(M * i) * zstride) : make_float2(0.0f, 0.0f);
-    for (int i = threadIdx.x; i < N; i += G::kThreads) w[i] = wN[i];
+            for (int i = 0; i < kZPoints; ++i)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                 unsigned(__cvta_generic_to_shared(stage + i * G::kThreads))),
+                             "l"(src + int64_t(M * i) * plane)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(blockIdx.x);
+    for (int i = threadIdx.x; i < N; i += G::kThreads) {
+        w[i] = wN[(i / M) * (i % M)];   // k1 n2 < N
+        T[i] = kphi.T[i] * kphi.scale;
+        if (kphi.M) D[i] = kphi.M[i];
+    }
     __syncthreads();
-    dft_dif<32, false>(a);   // a[i] = Y[k1 = brev(i)] of n2 = t
+    for (int tile = blockIdx.x; tile < kTiles; tile += gridDim.x) {
+        float2 a[kZPoints];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 1; i < kZPoints; ++i) a[i] = cmul(a[i], w[(t * brev<32>(i)) & (N - 1)]);
-    zexchange<N, true>(a, area, q, t);
-    dft_dif<M, false>(a);    // a[j M + i] = X[k1 + 32 brev(i)], k1 = J t + j
-    const typename KPhi::Pencil kp = kphi.pencil(active ? kx : 0, ky);
+        for (int i = 0; i < kZPoints; ++i) a[i] = stage[i * G::kThreads];
+        dft_dif<32, false>(a);   // a[i] = Y[k1 = brev(i)] of n2 = t
+        fetch(tile + gridDim.x); // the slots have been read: the transform above depends on them
 #pragma unroll
-    for (int i = 0; i < kZPoints; ++i) {
-        const float K = kphi.at(kp, J * t + i / M + 32 * brev<M>(i % M));
-        a[i] = make_float2(a[i].x * K, a[i].y * K);
+        for (int i = 1; i < kZPoints; ++i) a[i] = cmul(a[i], w[brev<32>(i) * M + t]);
+        zexchange<N, true>(a, area, q, t);
+        dft_dif<M, false>(a);    // a[j M + i] = X[k1 + 32 brev(i)], k1 = J t + j
+        const int pencil = tile * kZPencils + q, ky = pencil / nh, kx = pencil - ky * nh;
+        const typename KPhi::Pencil kp = kphi.pencil(kx, ky, T, D);
+#pragma unroll
+        for (int i = 0; i < kZPoints; ++i) {
+            const float K = kphi.at(kp, J * t + i / M + 32 * brev<M>(i % M), T, D);
+            a[i] = make_float2(a[i].x * K, a[i].y * K);
+        }
+        dft_dit<M, true>(a);     // a[j M + n2]
+#pragma unroll
+        for (int i = 0; i < kZPoints; ++i)
+            if (i % M != 0) a[i] = cmulc(a[i], w[J * t * M + i]);   // k1 M + n2
+        zexchange<N, false>(a, area, q, t);
+        dft_dit<32, true>(a);    // a[i] = x[t + M i]
+        float2* const dst = f + int64_t(tile) * kZPencils + q + t * plane;
+#pragma unroll
+        for (int i = 0; i < kZPoints; ++i) __stcs(dst + int64_t(M * i) * plane, a[i]);
     }
-    dft_dit<M, true>(a);     // a[j M + n2]
-#pragma unroll
-    for (int i = 0; i < kZPoints; ++i)
-        if (i % M != 0) a[i] = cmulc(a[i], w[((i % M) * (J * t + i / M)) & (N - 1)]);
-    zexchange<N, false>(a, area, q, t);
-    dft_dit<32, true>(a);    // a[i] = x[t + M i]
-    if (active) {
-#pragma unroll
-        for (int i = 0; i < kZPoints; ++i) __stcs(col + int64_t(M * i) * zstride, a[i]);
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 }  // namespace djb
