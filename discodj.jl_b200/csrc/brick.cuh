@@ -222,9 +222,14 @@ __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_SCATTER_BLOCKS) k_scat
             const unsigned slot = r0 + unsigned((tid & 31) * (kTileThreads / 32) + (tid >> 5));
             if (slot >= cnt) continue;
             const int64_t p = bl.perm[start + slot];
-            int i, j, k;
-            ld.ijk(p, i, j, k);
-            const float X[3] = {psi[p] + q1[i], psi[p + np] + q1[j], psi[p + 2 * np] + q1[k]};
+            float X[3] = {psi[p], psi[p + np], psi[p + 2 * np]};
+            if (q1) {   // else psi holds positions (resampled particle sets)
+                int i, j, k;
+                ld.ijk(p, i, j, k);
+                X[0] += q1[i];
+                X[1] += q1[j];
+                X[2] += q1[k];
+            }
 #pragma unroll 1
             for (int gb = 0; gb < NB; ++gb) {
                 const int g = g0 + gb;

@@ -48,9 +48,18 @@ constexpr int kMaxBins = 1024;
     } while (0)
 
 // Shell sums: sums[4*b + 0] = Σ w·P, [1] = Σ w, [2] = Σ |k|, counts[b] = modes.
+//
+// The modes (kx, ±ky, ±kz) share |k|, so a thread takes one kx and one |kz| and walks |ky|
+// upwards through `seg` of its res/2 + 1 values, four modes (the rows iy, res - iy of the
+// planes iz, res - iz) per square root. |k| then only grows along the walk: the sums stay
+// in registers while the shell is the same and go to shared memory when it ends, a few
+// times per walk. (One mode per thread with four shared float64 atomics each, most of them
+// on the same few shells, took 616 us at 256^3; this walk is bound by its loads.)
+// Lanes take consecutive kx, so a warp reads whole rows' stretches.
+constexpr int kShellAhead = 4;   // steps of the walk loaded together
 __global__ void __launch_bounds__(kThreads) k_shells(const float2* __restrict__ f, int res, double dk,
                                                       double norm, const double* __restrict__ edges,
-                                                      int bins, double* __restrict__ sums,
+                                                      int bins, int seg, double* __restrict__ sums,
                                                       unsigned long long* __restrict__ counts) {
     extern __shared__ double sm[];
     double* s_wp = sm;
@@ -65,33 +74,77 @@ __global__ void __launch_bounds__(kThreads) k_shells(const float2* __restrict__ 
     }
     __syncthreads();
     const int nh = res / 2 + 1;
-    const int64_t total = int64_t(res) * res * nh;
-    const double kmin = edges[0], kmax = edges[bins];
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
-         t += int64_t(gridDim.x) * blockDim.x) {
-        const int kx = int(t % nh);
-        const int iy = int((t / nh) % res);
-        const int iz = int(t / (int64_t(nh) * res));
+    const int chunks = (nh + 31) / 32;        // 32 kx per warp
+    const int nseg = (nh + seg - 1) / seg;
+    const int64_t items = int64_t(chunks) * nh * nseg;
+    const int64_t warps = int64_t(gridDim.x) * (kThreads / 32);
+    const double kmin = __ldg(edges), kmax = __ldg(edges + bins);
+    for (int64_t item = int64_t(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32; item < items; item += warps) {
+        const int kx = int(item % chunks) * 32 + (threadIdx.x & 31);
+        if (kx >= nh) continue;
+        const int jz = int((item / chunks) % nh);
+        const int y0 = int(item / (int64_t(chunks) * nh)) * seg, y1 = min(y0 + seg, nh);
         // full axes: index <= res/2 positive (power_spectrum.jl:40)
-        const double ky = double(iy <= res / 2 ? iy : iy - res) * dk;
-        const double kz = double(iz <= res / 2 ? iz : iz - res) * dk;
-        const double kh = double(kx) * dk;
-        // same association as the reference's kx²+ky²+kz² with its halved axis last
-        const double k = sqrt((kz * kz + ky * ky) + kh * kh);
-        if (!(k >= kmin && k < kmax)) continue;
-        int lo = 0, hi = bins;  // edges[lo] <= k < edges[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (edges[mid] <= k) lo = mid;
-            else hi = mid;
-        }
-        const float2 v = f[t];
-        const double p = (double(v.x) * v.x + double(v.y) * v.y) * norm;
+        const bool two_z = jz > 0 && 2 * jz < res;
+        const float2* const p0 = f + int64_t(jz) * res * nh + kx;
+        const float2* const p1 = f + int64_t(two_z ? res - jz : jz) * res * nh + kx;
+        const double kz = double(jz) * dk, kh = double(kx) * dk;
+        const double kz2 = kz * kz, kh2 = kh * kh;
         const double w = (kx == 0 || kx == nh - 1) ? 0.5 : 1.0;
-        atomicAdd(&s_wp[lo], w * p);
-        atomicAdd(&s_w[lo], w);
-        atomicAdd(&s_k[lo], k);
-        atomicAdd(&s_n[lo], 1ull);
+        int lo = 0;                              // shell of the running sums: [elo, ehi)
+        double elo = kmin, ehi = __ldg(edges + 1), sp = 0.0, sk = 0.0;
+        unsigned cnt = 0;
+        const auto flush = [&]() {
+            if (cnt) {
+                atomicAdd(&s_wp[lo], w * sp);
+                atomicAdd(&s_w[lo], w * double(cnt));
+                atomicAdd(&s_k[lo], sk);
+                atomicAdd(&s_n[lo], (unsigned long long)cnt);
+            }
+            sp = sk = 0.0;
+            cnt = 0;
+        };
+        for (int jy = y0; jy < y1; jy += kShellAhead) {
+            float2 v[kShellAhead][4];
+#pragma unroll
+            for (int u = 0; u < kShellAhead; ++u) {
+                const int j = min(jy + u, y1 - 1), jm = (j > 0 && 2 * j < res) ? res - j : j;
+                v[u][0] = __ldcs(p0 + int64_t(j) * nh);
+                v[u][1] = __ldcs(p0 + int64_t(jm) * nh);
+                v[u][2] = __ldcs(p1 + int64_t(j) * nh);
+                v[u][3] = __ldcs(p1 + int64_t(jm) * nh);
+            }
+#pragma unroll
+            for (int u = 0; u < kShellAhead; ++u) {
+                const int j = jy + u;
+                if (j >= y1) break;
+                const double ky = double(j) * dk;
+                // same association as the reference's kx²+ky²+kz² with its halved axis last
+                const double k = sqrt((kz2 + ky * ky) + kh2);
+                if (!(k >= kmin && k < kmax)) continue;
+                if (!(k >= elo && k < ehi)) {   // the walk enters another shell
+                    flush();
+                    int a = (k >= elo) ? lo : 0, z = bins;   // edges[a] <= k < edges[z]
+                    while (z - a > 1) {
+                        const int mid = (a + z) >> 1;
+                        if (__ldg(edges + mid) <= k) a = mid;
+                        else z = mid;
+                    }
+                    lo = a;
+                    elo = __ldg(edges + a);
+                    ehi = __ldg(edges + a + 1);
+                }
+                const bool two_y = j > 0 && 2 * j < res;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    if (((m & 1) && !two_y) || ((m & 2) && !two_z)) continue;
+                    sp += (double(v[u][m].x) * v[u][m].x + double(v[u][m].y) * v[u][m].y) * norm;
+                    sk += k;
+                    ++cnt;
+                }
+            }
+        }
+        flush();
     }
     __syncthreads();
     for (int b = threadIdx.x; b < bins; b += blockDim.x) {
@@ -101,6 +154,22 @@ __global__ void __launch_bounds__(kThreads) k_shells(const float2* __restrict__ 
         atomicAdd(&sums[4 * b + 2], s_k[b]);
         atomicAdd(&counts[b], s_n[b]);
     }
+}
+
+// Launches k_shells: the walks are cut into segments until there are enough warps for every
+// SM (16 each), and the grid never exceeds what is resident, so that the per-block sums are
+// merged a bounded number of times.
+cudaError_t launch_shells(const float2* spec, int res, double dk, double norm, const double* edges, int bins,
+                          double* sums, unsigned long long* counts, cudaStream_t st) {
+    const int nh = res / 2 + 1;
+    const int64_t strips = int64_t((nh + 31) / 32) * nh;
+    int seg = nh;
+    while (seg > 16 && strips * ((nh + seg - 1) / seg) < 148 * 16) seg = (seg + 1) / 2;
+    const int64_t items = strips * ((nh + seg - 1) / seg);
+    const int grid = int(std::min<int64_t>((items + kThreads / 32 - 1) / (kThreads / 32), 148 * 4));
+    k_shells<<<grid, kThreads, size_t(bins) * 4 * sizeof(double), st>>>(spec, res, dk, norm, edges, bins, seg, sums,
+                                                                       counts);
+    return cudaGetLastError();
 }
 
 // spec[k] *= coef[bin(k)] (0 outside every bin): the bins of k_shells.
@@ -188,11 +257,7 @@ int shells(const float2* spec, int res, double boxsize, double scale2, int bins,
         const double V = boxsize * boxsize * boxsize;
         const double r3 = double(res) * res * res;
         const double norm = V / (r3 * r3) * scale2;
-        const int64_t total = int64_t(res) * res * (res / 2 + 1);
-        int grid = int(std::min<int64_t>((total + kThreads - 1) / kThreads, 148 * 8));
-        const size_t smem = size_t(bins) * 4 * sizeof(double);
-        k_shells<<<grid, kThreads, smem, st>>>(spec, res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums, d_counts);
-        cudaError_t le = cudaGetLastError();
+        const cudaError_t le = launch_shells(spec, res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums, d_counts, st);
         if (le != cudaSuccess) {
             rc = fail(DJB_ERR_CUDA, "shell kernel launch failed: %s", cudaGetErrorString(le));
             break;
@@ -346,11 +411,8 @@ int djb_power_spectrum_shells_noalloc(const void* spectrum, int32_t res, double 
     const double V = boxsize * boxsize * boxsize;
     const double r3 = double(res) * res * res;
     const double norm = V / (r3 * r3) * scale2;
-    const int64_t total = int64_t(res) * res * (res / 2 + 1);
-    const int grid = int(std::min<int64_t>((total + kThreads - 1) / kThreads, 148 * 8));
-    k_shells<<<grid, kThreads, size_t(bins) * 4 * sizeof(double), st>>>(
-        static_cast<const float2*>(spectrum), res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums, d_counts);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_shells(static_cast<const float2*>(spectrum), res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums,
+                           d_counts, st));
     CUDA_TRY(cudaMemcpyAsync(sums, d_sums, sizeof(double) * 4 * bins, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(counts, d_counts, sizeof(unsigned long long) * bins, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));

@@ -605,11 +605,11 @@ __global__ void k_output(const float* __restrict__ psi, const float* __restrict_
 // ── sheet resampling (pm.jl:186-234,426-464) ──────────────────────────────────
 // ψ_c = mod(X_c + s_c - q_c + L/2, L) - L/2 with X = q + Psi, written transposed to
 // [i][j][k] (k fastest, row padded to n+2) so that the in-place R2C halves the z
-// axis as the reference's rfft does (pm.jl:430-433).
+// axis as the reference's rfft does (pm.jl:430-433). blockIdx.y: the component; `out`
+// holds the three of them `ostride` floats apart.
 __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restrict__ q1, int n,
-                           int64_t np, float L, Shift3 s, int c, float* __restrict__ out,
-                           int padded) {
-    const int pitch = padded ? n + 2 : n;
+                           int64_t np, float L, Shift3 s, float* __restrict__ out, int64_t ostride) {
+    const int pitch = n + 2, c = blockIdx.y;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < np;
          t += int64_t(gridDim.x) * blockDim.x) {
         // t enumerates the output in [i][j][k] order (k fastest)
@@ -621,7 +621,7 @@ __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restric
         const int qi = (c == 0) ? ii : (c == 1) ? jj : kk;
         const float X = (psi[p + c * np] + q1[qi]) + sc;
         const float v = jmodf((X - q1[qi]) + L / 2.0f, L) - L / 2.0f;
-        out[(int64_t(ii) * n + jj) * pitch + kk] = v;
+        out[c * ostride + (int64_t(ii) * n + jj) * pitch + kk] = v;
     }
 }
 
@@ -630,12 +630,14 @@ __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restric
 // kz = n/2 planes are made Hermitian ((H(k) + conj H(-k))/2), which is the value
 // a C2R that ignores the imaginary part of those planes after the full-axis
 // transforms produces from the raw product; it makes the result independent of
-// the C2R implementation.
+// the C2R implementation. blockIdx.y: the component (three spectra back to back).
 __global__ void k_phase(const float2* __restrict__ in, float2* __restrict__ out, int n,
                         const float2* __restrict__ px, const float2* __restrict__ py,
                         const float2* __restrict__ pz, float scale) {
     const int nh = n / 2 + 1;
     const int64_t total = int64_t(n) * n * nh;
+    in += blockIdx.y * total;
+    out += blockIdx.y * total;
     auto cmul = [](float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); };
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
          t += int64_t(gridDim.x) * blockDim.x) {
@@ -663,17 +665,18 @@ __global__ void k_phase(const float2* __restrict__ in, float2* __restrict__ out,
 
 // Resampled positions X' = mod(q + ψ' + d·L/n + L, L) for the Fourier method
 // (pm.jl:438-441), ψ' in [i][j][k] padded layout, written to xr (3 blocks of n³,
-// same [i][j][k] order).
-__global__ void k_place(const float* __restrict__ rb, const float* __restrict__ q1, int n,
-                        int64_t np, float L, float shiftc, int c, float* __restrict__ xr) {
-    const int pitch = n + 2;
+// same [i][j][k] order). blockIdx.y: the component.
+__global__ void k_place(const float* __restrict__ rb, int64_t rstride, const float* __restrict__ q1, int n,
+                        int64_t np, float L, Shift3 shift, float* __restrict__ xr) {
+    const int pitch = n + 2, c = blockIdx.y;
+    const float shiftc = (c == 0) ? shift.x : (c == 1) ? shift.y : shift.z;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < np;
          t += int64_t(gridDim.x) * blockDim.x) {
         const int kk = int(t % n);
         const int jj = int((t / n) % n);
         const int ii = int(t / (int64_t(n) * n));
         const int qi = (c == 0) ? ii : (c == 1) ? jj : kk;
-        const float v = rb[(int64_t(ii) * n + jj) * pitch + kk];
+        const float v = rb[c * rstride + (int64_t(ii) * n + jj) * pitch + kk];
         xr[t + c * np] = jmodf(((q1[qi] + v) + shiftc) + L, L);
     }
 }
@@ -890,8 +893,8 @@ struct djb_solver {
     float* gf = nullptr;
     // resampling work areas
     float2* psihat = nullptr;   // 3 spectra (n, n, n/2+1)
-    float2* cb = nullptr;       // one spectrum
-    float* rb = nullptr;        // real n*n*(n+2) (in-place C2R)
+    float2* cb = nullptr;       // 3 spectra
+    float* rb = nullptr;        // 3 real n*n*(n+2) arrays
     float* xr = nullptr;        // 3*np resampled positions
     float2* phase = nullptr;    // px, py, pz tables (n + n + n/2+1)
     // brick sort of the particles (sort.cuh)
@@ -905,6 +908,10 @@ struct djb_solver {
     unsigned* bsum = nullptr;
     uint2* keyrank = nullptr;
     int* perm = nullptr;
+    // the same for the resampled particle sets (one at a time)
+    unsigned* offset_r = nullptr;
+    unsigned* bsum_r = nullptr;
+    int* perm_r = nullptr;
     float* part = nullptr;  // brick interpolation's partial sums and Ψ in sorted order (6 np floats), or null
     const int* cur_perm = nullptr;  // order used by the tiled kernels of the current force call
     int* err = nullptr;
@@ -989,7 +996,7 @@ int validate(const djb_pm_config& c) {
     return DJB_OK;
 }
 
-int make_plan(cufftHandle* h, bool* have, int n, cufftType type, cudaStream_t st, size_t* work) {
+int make_plan(cufftHandle* h, bool* have, int n, cufftType type, cudaStream_t st, size_t* work, int batch = 1) {
     CUFFT_TRY(cufftCreate(h));
     *have = true;
     long long dims[3] = {n, n, n};
@@ -1000,7 +1007,7 @@ int make_plan(cufftHandle* h, bool* have, int n, cufftType type, cudaStream_t st
     long long* onembed = fwd ? cembed : rembed;
     long long idist = inembed[0] * inembed[1] * inembed[2];
     long long odist = onembed[0] * onembed[1] * onembed[2];
-    CUFFT_TRY(cufftMakePlanMany64(*h, 3, dims, inembed, 1, idist, onembed, 1, odist, type, 1, work));
+    CUFFT_TRY(cufftMakePlanMany64(*h, 3, dims, inembed, 1, idist, onembed, 1, odist, type, batch, work));
     CUFFT_TRY(cufftSetStream(*h, st));
     return DJB_OK;
 }
@@ -1164,6 +1171,39 @@ void launch_scatter_positions(djb_solver* s, const float* xr, int64_t count, flo
     if (s->W == 4) djb::k_scatter_positions<4><<<b, kThreads, 0, s->stream>>>(xr, count, count, s->Lf, s->res, pitch, mesh, s->err);
 }
 
+// Deposit of n³ given positions (a resampled particle set) into `mesh`: sorted by brick
+// and added by the brick kernel, with sort arrays of its own (the force's order stays valid
+// for its interpolation); without the sort, one thread per particle with float atomics on
+// the mesh. At 96³ particles / 192³ mesh (PCS): see resample_deposit.
+int scatter_positions(djb_solver* s, const float* xr, float* mesh, int pitch) {
+    if (!(s->tiled && s->sorted && s->perm_r)) {
+        launch_scatter_positions(s, xr, s->np, mesh, pitch);
+        return DJB_OK;
+    }
+    CUDA_TRY(cudaMemsetAsync(s->count, 0, size_t(s->nbins) * sizeof(unsigned), s->stream));
+    djb::k_bin<<<blocks(s->np), 256, 0, s->stream>>>(const_cast<float*>(xr), nullptr, 0.0f, nullptr, s->n, s->np, s->Lf,
+                                                      s->sg, s->count, s->keyrank, s->err);
+    djb::k_scan_block<<<s->nscan, djb::kScanThreads, 0, s->stream>>>(s->count, s->nbins, s->offset_r, s->bsum_r);
+    djb::k_scan_sums<<<1, djb::kScanThreads, 0, s->stream>>>(s->bsum_r, s->nscan);
+    djb::k_place<<<blocks(s->np), 256, 0, s->stream>>>(s->keyrank, s->np, s->offset_r, s->bsum_r, s->perm_r);
+    djb::BrickList bl = brick_list(s);
+    bl.offset = s->offset_r;
+    bl.bsum = s->bsum_r;
+    bl.perm = s->perm_r;
+    const unsigned nbricks = unsigned(s->sg.nb) * s->sg.nb * s->sg.nb;
+    const int tma = (s->tma && mesh == s->phi[0]) ? 1 : 0;
+    const GroupShifts none{};   // a shift of 0 lies inside the box of every configuration
+#define DJB_SP(W_)                                                                                              \
+    if (s->W == W_)                                                                                             \
+        djb::k_scatter_brick<W_, 1><<<nbricks, djb::kTileThreads, scatter_smem(s), s->stream>>>(                 \
+            xr, nullptr, s->n, s->np, s->Lf, s->res, pitch, none, mesh, nullptr, s->err, bl, s->tmap_s[0],      \
+            s->tmap_s[0], tma);
+    DJB_SP(2) DJB_SP(3) DJB_SP(4)
+#undef DJB_SP
+    CUDA_TRY(cudaGetLastError());
+    return DJB_OK;
+}
+
 template <int W, int R>
 void launch_gather_wr(djb_solver* s, const djb::GatherArgs& a, int ns) {
     if (R > 0 && s->tiled && a.perm) {
@@ -1276,23 +1316,22 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
     const int64_t nreal = int64_t(n) * n * (n + 2);
     const int nof = int(s->rshifts.size() / 3);
     if (s->cfg.resampling == DJB_RESAMPLE_FOURIER) {
-        for (int c = 0; c < 3; ++c) {
-            djb::k_wrap_psi<<<grid_for(np), kThreads, 0, s->stream>>>(s->psi, s->q1, n, np, s->Lf, sh, c, s->rb, 1);
-            CUFFT_TRY(cufftExecR2C(s->r2c_n, s->rb, reinterpret_cast<cufftComplex*>(s->psihat + c * nspec)));
-        }
+        // the three components of a set go through each kernel and transform together (a
+        // component alone is launch-sized at the usual 64³-128³ particles)
+        const dim3 gp(unsigned(grid_for(np)), 3), gs(unsigned(grid_for(nspec)), 3);
+        djb::k_wrap_psi<<<gp, kThreads, 0, s->stream>>>(s->psi, s->q1, n, np, s->Lf, sh, s->rb, nreal);
+        CUFFT_TRY(cufftExecR2C(s->r2c_n, s->rb, reinterpret_cast<cufftComplex*>(s->psihat)));
         for (int o = 0; o < nof; ++o) {
-            const double d[3] = {s->rshifts[3 * o], s->rshifts[3 * o + 1], s->rshifts[3 * o + 2]};
+            const double* d = &s->rshifts[3 * o];
             const float2* px = s->phase + int64_t(o) * (2 * n + nh);
-            for (int c = 0; c < 3; ++c) {
-                djb::k_phase<<<grid_for(nspec), kThreads, 0, s->stream>>>(
-                    s->psihat + c * nspec, s->cb, n, px, px + n, px + 2 * n, float(1.0 / (double(n) * n * n)));
-                CUFFT_TRY(cufftExecC2R(s->c2r_n, reinterpret_cast<cufftComplex*>(s->cb), s->rb));
-                djb::k_place<<<grid_for(np), kThreads, 0, s->stream>>>(
-                    s->rb, s->q1, n, np, s->Lf, float(d[c] * s->cfg.boxsize / n), c, s->xr);
-            }
-            launch_scatter_positions(s, s->xr, np, mesh, rho_pitch(s));
+            djb::k_phase<<<gs, kThreads, 0, s->stream>>>(s->psihat, s->cb, n, px, px + n, px + 2 * n,
+                                                         float(1.0 / (double(n) * n * n)));
+            CUFFT_TRY(cufftExecC2R(s->c2r_n, reinterpret_cast<cufftComplex*>(s->cb), s->rb));
+            const Shift3 off{float(d[0] * s->cfg.boxsize / n), float(d[1] * s->cfg.boxsize / n),
+                             float(d[2] * s->cfg.boxsize / n)};
+            djb::k_place<<<gp, kThreads, 0, s->stream>>>(s->rb, nreal, s->q1, n, np, s->Lf, off, s->xr);
+            TRY(scatter_positions(s, s->xr, mesh, rho_pitch(s)));
         }
-        (void)nreal;
     } else {
         djb::k_wrap_psi_lin<<<grid_for(3 * np), kThreads, 0, s->stream>>>(s->psi, s->q1, n, np, s->Lf, sh, s->rb);
         for (int o = 0; o < nof; ++o) {
@@ -1301,7 +1340,7 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
                 s->rb, s->q1, n, np, s->Lf, float(d[0]), float(d[1]), float(d[2]),
                 float(d[0] * s->cfg.boxsize / n), float(d[1] * s->cfg.boxsize / n),
                 float(d[2] * s->cfg.boxsize / n), s->xr);
-            launch_scatter_positions(s, s->xr, np, mesh, rho_pitch(s));
+            TRY(scatter_positions(s, s->xr, mesh, rho_pitch(s)));
         }
     }
     return DJB_OK;
@@ -1939,11 +1978,16 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
     if (resample) {
         const int n = s->n, nh = n / 2 + 1;
         const int64_t nspec = int64_t(n) * n * nh;
-        TRY(dmalloc(s, (void**)&s->rb, sizeof(float) * std::max<int64_t>(int64_t(n) * n * (n + 2), 3 * s->np)));
+        TRY(dmalloc(s, (void**)&s->rb, sizeof(float) * 3 * size_t(n) * n * (n + 2)));
         TRY(dmalloc(s, (void**)&s->xr, pbytes));
+        if (s->sorted) {
+            TRY(dmalloc(s, (void**)&s->offset_r, sizeof(unsigned) * size_t(s->nbins)));
+            TRY(dmalloc(s, (void**)&s->bsum_r, sizeof(unsigned) * size_t(s->nscan)));
+            TRY(dmalloc(s, (void**)&s->perm_r, sizeof(int) * size_t(s->np)));
+        }
         if (cfg->resampling == DJB_RESAMPLE_FOURIER) {
             TRY(dmalloc(s, (void**)&s->psihat, sizeof(float2) * 3 * nspec));
-            TRY(dmalloc(s, (void**)&s->cb, sizeof(float2) * nspec));
+            TRY(dmalloc(s, (void**)&s->cb, sizeof(float2) * 3 * nspec));
             // phase tables exp(2πi m d/n) per offset (pm.jl:453-456); full axes hold
             // -n/2 at index n/2, the halved axis m/n for m = 0..n/2
             const int nof = int(s->rshifts.size() / 3);
@@ -1963,9 +2007,9 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             }
             TRY(dmalloc(s, (void**)&s->phase, sizeof(float2) * h.size()));
             CUDA_TRY(cudaMemcpy(s->phase, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
-            TRY(make_plan(&s->r2c_n, &s->have_r2c_n, n, CUFFT_R2C, s->stream, &work));
+            TRY(make_plan(&s->r2c_n, &s->have_r2c_n, n, CUFFT_R2C, s->stream, &work, 3));
             s->bytes += int64_t(work);
-            TRY(make_plan(&s->c2r_n, &s->have_c2r_n, n, CUFFT_C2R, s->stream, &work));
+            TRY(make_plan(&s->c2r_n, &s->have_c2r_n, n, CUFFT_C2R, s->stream, &work, 3));
             s->bytes += int64_t(work);
         }
     }
