@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -27,6 +28,7 @@ cufftHandle solver_c2r(const djb_solver* s);
 double solver_boxsize(const djb_solver* s);
 int solver_cic_gather_grad(djb_solver* s, const float* mesh, int pitch, float* psibar);
 int solver_check_err(djb_solver* s);
+int solver_shell_area(djb_solver* s, size_t bytes, void** area);
 }  // namespace djb
 
 namespace {
@@ -225,54 +227,34 @@ std::vector<double> bin_edges(int res, double boxsize, int bins, bool logarithmi
     return e;
 }
 
-// Bins the spectrum `spec` (already transformed) and writes k, P, N on the host.
+// Device work area of the shell sums: bins + 1 edges, 4 bins sums, bins counts.
+size_t shell_area_bytes(int bins) { return sizeof(double) * (6 * size_t(bins) + 1); }
+
+// Bins the spectrum `spec` (already transformed) and writes k, P, N on the host. d_area:
+// shell_area_bytes(bins) of device memory. Edges and cleared sums go up in one copy, sums
+// and counts come back in one.
 int shells(const float2* spec, int res, double boxsize, double scale2, int bins, bool logarithmic,
-           double* k_out, double* pk_out, int64_t* n_out, cudaStream_t st, double* wsum_out = nullptr) {
-    std::vector<double> e = bin_edges(res, boxsize, bins, logarithmic);
-    double* d_edges = nullptr;
-    double* d_sums = nullptr;
-    unsigned long long* d_counts = nullptr;
-    int rc = DJB_OK;
-    auto cleanup = [&]() {
-        if (d_edges) cudaFreeAsync(d_edges, st);
-        if (d_sums) cudaFreeAsync(d_sums, st);
-        if (d_counts) cudaFreeAsync(d_counts, st);
-    };
-    if (cudaMallocAsync((void**)&d_edges, sizeof(double) * (bins + 1), st) != cudaSuccess ||
-        cudaMallocAsync((void**)&d_sums, sizeof(double) * 4 * bins, st) != cudaSuccess ||
-        cudaMallocAsync((void**)&d_counts, sizeof(unsigned long long) * bins, st) != cudaSuccess) {
-        cudaGetLastError();
-        cleanup();
-        return fail(DJB_ERR_ALLOC, "power spectrum work area allocation failed");
-    }
-    std::vector<double> sums(4 * size_t(bins));
-    std::vector<unsigned long long> counts(bins);
-    do {
-        if (cudaMemcpyAsync(d_edges, e.data(), sizeof(double) * (bins + 1), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-            cudaMemsetAsync(d_sums, 0, sizeof(double) * 4 * bins, st) != cudaSuccess ||
-            cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * bins, st) != cudaSuccess) {
-            rc = fail(DJB_ERR_CUDA, "power spectrum set-up copy failed");
-            break;
-        }
-        const double V = boxsize * boxsize * boxsize;
-        const double r3 = double(res) * res * res;
-        const double norm = V / (r3 * r3) * scale2;
-        const cudaError_t le = launch_shells(spec, res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums, d_counts, st);
-        if (le != cudaSuccess) {
-            rc = fail(DJB_ERR_CUDA, "shell kernel launch failed: %s", cudaGetErrorString(le));
-            break;
-        }
-        if (cudaMemcpyAsync(sums.data(), d_sums, sizeof(double) * 4 * bins, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaMemcpyAsync(counts.data(), d_counts, sizeof(unsigned long long) * bins, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
-            rc = fail(DJB_ERR_CUDA, "power spectrum read-back failed");
-            break;
-        }
-    } while (false);
-    cleanup();
-    if (rc != DJB_OK) return rc;
+           double* k_out, double* pk_out, int64_t* n_out, cudaStream_t st, void* d_area, double* wsum_out = nullptr) {
+    const std::vector<double> e = bin_edges(res, boxsize, bins, logarithmic);
+    std::vector<double> h(6 * size_t(bins) + 1, 0.0);
+    std::copy(e.begin(), e.end(), h.begin());
+    double* const d_edges = static_cast<double*>(d_area);
+    double* const d_sums = d_edges + bins + 1;
+    unsigned long long* const d_counts = reinterpret_cast<unsigned long long*>(d_sums + 4 * bins);
+    if (cudaMemcpyAsync(d_area, h.data(), shell_area_bytes(bins), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        return fail(DJB_ERR_CUDA, "power spectrum set-up copy failed");
+    const double V = boxsize * boxsize * boxsize;
+    const double r3 = double(res) * res * res;
+    const double norm = V / (r3 * r3) * scale2;
+    const cudaError_t le = launch_shells(spec, res, 2 * M_PI / boxsize, norm, d_edges, bins, d_sums, d_counts, st);
+    if (le != cudaSuccess) return fail(DJB_ERR_CUDA, "shell kernel launch failed: %s", cudaGetErrorString(le));
+    if (cudaMemcpyAsync(h.data(), d_sums, sizeof(double) * 5 * bins, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return fail(DJB_ERR_CUDA, "power spectrum read-back failed");
+    const double* const sums = h.data();
     for (int b = 0; b < bins; ++b) {
-        const unsigned long long n = counts[b];
+        unsigned long long n;
+        std::memcpy(&n, h.data() + 4 * size_t(bins) + b, sizeof(n));
         if (wsum_out) wsum_out[b] = sums[4 * b + 1];
         if (n == 0) {
             k_out[b] = std::sqrt(e[b] * e[b + 1]);
@@ -442,11 +424,13 @@ int djb_power_spectrum(const float* field, int32_t res, double boxsize, int32_t 
     CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     const int pitch = res + 2;
     float* mesh = nullptr;
+    void* area = nullptr;
     cufftHandle plan = 0;
     bool have_plan = false;
     int rc = DJB_OK;
     do {
-        if (cudaMallocAsync((void**)&mesh, sizeof(float) * size_t(res) * res * pitch, st) != cudaSuccess) {
+        if (cudaMallocAsync((void**)&mesh, sizeof(float) * size_t(res) * res * pitch, st) != cudaSuccess ||
+            cudaMallocAsync(&area, shell_area_bytes(bins), st) != cudaSuccess) {
             cudaGetLastError();
             rc = fail(DJB_ERR_ALLOC, "power spectrum mesh allocation failed");
             break;
@@ -476,9 +460,10 @@ int djb_power_spectrum(const float* field, int32_t res, double boxsize, int32_t 
             break;
         }
         rc = shells(reinterpret_cast<const float2*>(mesh), res, boxsize, 1.0, bins, logarithmic != 0, k, pk,
-                    nmodes, st);
+                    nmodes, st, area);
     } while (false);
     if (have_plan) cufftDestroy(plan);
+    if (area) cudaFreeAsync(area, st);
     if (mesh) cudaFreeAsync(mesh, st);
     cudaStreamSynchronize(st);
     cudaStreamDestroy(st);
@@ -498,8 +483,11 @@ int djb_state_power_spectrum(djb_solver* s, int32_t bins, int32_t logarithmic, d
     CUFFT_TRY(cufftExecR2C(djb::solver_r2c(s), mesh, reinterpret_cast<cufftComplex*>(mesh)));
     // δ = mesh·res³/n³ − 1: for k ≠ 0 the spectrum scales by (res³/n³)²
     const double f = double(res) * res * res / double(djb::solver_np(s));
+    void* area = nullptr;
+    rc = djb::solver_shell_area(s, shell_area_bytes(bins), &area);
+    if (rc != DJB_OK) return rc;
     return shells(reinterpret_cast<const float2*>(mesh), res, djb::solver_boxsize(s), f * f, bins,
-                  logarithmic != 0, k, pk, nmodes, st);
+                  logarithmic != 0, k, pk, nmodes, st, area);
 }
 
 int djb_state_density_modes(djb_solver* s, int32_t nmodes, const int32_t* modes, double* out) {
@@ -563,8 +551,11 @@ int djb_state_power_spectrum_vjp(djb_solver* s, int32_t bins, int32_t logarithmi
     const double f = double(res) * res * res / double(djb::solver_np(s));
     std::vector<double> kk(bins), pk(bins), wsum(bins), coef(bins);
     std::vector<int64_t> nm(bins);
+    void* area = nullptr;
+    rc = djb::solver_shell_area(s, shell_area_bytes(bins), &area);
+    if (rc != DJB_OK) return rc;
     rc = shells(reinterpret_cast<const float2*>(mesh), res, boxsize, f * f, bins, logarithmic != 0, kk.data(),
-                pk.data(), nm.data(), st, wsum.data());
+                pk.data(), nm.data(), st, area, wsum.data());
     if (rc != DJB_OK) return rc;
     const double V = boxsize * boxsize * boxsize;
     const double r3 = double(res) * res * res;

@@ -353,3 +353,29 @@ def test_sorted_partial_sums_change_no_bit(djb, monkeypatch, W, g, aa):
             out[mode] = (acc, *S.output(wrap=False))
     for a, b in zip(out["0"], out["1"]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("grad,aa", [(4, 0), (4, 2), (0, 1), (0, 2)])
+def test_acceleration_in_place_and_resident_state(djb, grad, aa):
+    """A force on device arrays reads the displacements where they are: the result may
+    overwrite them (the same bits as with an array of its own, up to the order of the
+    deposit's float reductions), and the resident state stays what it was."""
+    import torch
+    n, res, L = 12, 24, 30.0
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    psi = 0.7 * torch.randn((3, n, n, n), generator=gen, device="cuda")
+    mom = torch.randn((3, n, n, n), generator=gen, device="cuda")
+    keep = psi.clone()
+    with djb.PMSolver(djb.PMConfig(res_pm=res, n_part=n, boxsize=L, worder=3, grad_order=grad, antialias=aa)) as S:
+        S.set_state(mom, psi)
+        torch.cuda.synchronize()
+        a = S.acceleration(psi)
+        assert torch.equal(psi, keep)
+        both = psi.clone()
+        torch.cuda.synchronize()
+        S.acceleration(both, out=both)
+        assert rel(both.cpu().numpy(), a.cpu().numpy()) < 1e-5
+        h = S.acceleration(djb.logical_view(psi).cpu().numpy())
+        assert rel(h, djb.logical_view(a).cpu().numpy()) < 1e-5
+        p, m = S.get_state(device=True)
+        assert torch.equal(p, mom) and torch.equal(m, psi)
