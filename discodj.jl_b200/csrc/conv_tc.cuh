@@ -17,7 +17,7 @@
 //     tensor copy per plane (5-D map over [z][chunk][y][x][8 channels]) where the halo
 //     does not wrap, else 16-byte cp.async with the periodic wrap; completion on the
 //     slot's `full` barrier.
-//   MMA (warp 9, converged; one elected lane issues): per plane, tcgen05.mma of
+//   MMA (warp 9; one elected lane runs the loop): per plane, tcgen05.mma of
 //     128 × N·(tiles it feeds) × 16 (bf16 operands, float32 accumulation) per
 //     (dy, dx, K step); commits to the `empty` barrier of the plane and to the `accf`
 //     barrier of the tile the plane completes.
@@ -109,11 +109,9 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
 }
 
-// Instruction descriptor of kind::f16: bf16 A and B (K-major), float32 D, M = 128.
-template <int N>
-__device__ __forceinline__ uint32_t idesc() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
+// Instruction descriptor of kind::f16: bf16 A and B (K-major), float32 D, M = 128; the N
+// field, (n >> 3) << 17, is filled in per MMA.
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(128 >> 4) << 24);
 
 __device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
     asm volatile(
@@ -132,26 +130,6 @@ __device__ __forceinline__ void mma_bf16_w(uint32_t dtmem, uint32_t alo, uint32_
         " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(dtmem),
         "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(id), "r"(acc)
-        : "memory");
-}
-
-// The same, executed by the whole converged warp: one lane, chosen by elect.sync inside
-// the instruction sequence, issues it; the operands stay warp-uniform.
-__device__ __forceinline__ void mma_bf16_warp(uint32_t dtmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
-                                              uint32_t id, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p, e;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n"
-        " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n elect.sync _|e, 0xffffffff;\n"
-        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}" ::"r"(dtmem),
-        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(id), "r"(acc)
-        : "memory");
-}
-
-// tcgen05.commit by one elected lane of the converged warp.
-__device__ __forceinline__ void mma_commit_warp(uint64_t* bar) {
-    asm volatile(
-        "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
-        " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar))
         : "memory");
 }
 
@@ -240,8 +218,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 
 // Bounded barrier wait of one role; false (and the CTA's abort flag set) when it ran
-// out or another role has aborted.
+// out or another role has aborted. A barrier that is ready costs one test: the flag and
+// the clock are read only when the role has to wait.
 __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    if (mbar_try(bar, parity)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar, parity)) return true;
     *abort_flag = 1;
@@ -363,6 +343,18 @@ __global__ void __launch_bounds__(kThreads, 1)
             const Item it = item_of(a, item);
             const bool interior = a.use_tma && it.x0 >= 1 && it.x0 - 1 + kBX <= a.res && it.y0 >= 1 &&
                                   it.y0 - 1 + kBY <= a.res;
+            // tiles whose halo wraps: this lane's offsets in a plane, the same for every plane
+            constexpr int kCopies = (CC * kPlane + 31) / 32;
+            int off[kCopies];
+            if (!interior) {
+#pragma unroll
+                for (int i = 0; i < kCopies; ++i) {
+                    const int e = min(lane + 32 * i, CC * kPlane - 1);
+                    const int pos = e / CC, by = pos / kBX, bx = pos - by * kBX;
+                    off[i] = (wrap(it.y0 - 1 + by, a.res) * a.res + wrap(it.x0 - 1 + bx, a.res)) * (CC * 8) +
+                             (e - pos * CC) * 8;
+                }
+            }
             for (int j = 0; j < it.nt + 2; ++j, ++k) {
                 const int slot = int(k % kRing);
                 if (!role_wait(&empty[slot], ((k / kRing) & 1u) ^ 1u, abort_flag)) {
@@ -379,13 +371,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                         mbar_arrive(&full[slot]);
                     }
                 } else {
-                    for (int e = lane; e < CC * kPlane; e += 32) {
-                        const int pos = e / CC, kc = e - pos * CC;
-                        const int by = pos / kBX, bx = pos - by * kBX;
-                        const int gy = wrap(it.y0 - 1 + by, a.res), gx = wrap(it.x0 - 1 + bx, a.res);
-                        const __nv_bfloat16* src =
-                            a.X + ((int64_t(gz) * a.res + gy) * a.res + gx) * (CC * 8) + kc * 8;
-                        cp_async16(dst + uint32_t((kc * kPlane + pos) * 16), src);
+                    const __nv_bfloat16* const src = a.X + int64_t(gz) * a.res * a.res * (CC * 8);
+#pragma unroll
+                    for (int i = 0; i < kCopies; ++i) {
+                        const int e = lane + 32 * i, pos = e / CC, kc = e - pos * CC;
+                        if (e < CC * kPlane) cp_async16(dst + uint32_t((kc * kPlane + pos) * 16), src + off[i]);
                     }
                     cp_async_arrive(&full[slot]);
                 }
@@ -400,75 +390,77 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp == kMmaWarp) {
         // ── MMA issue: per staged plane u (z0 − 1 .. z0 + L), one MMA per (shift, K step)
         // of N · (tiles it feeds): the plane is the kz = 0, 1, 2 input of tiles u + 1, u,
-        // u − 1, whose accumulators are adjacent; the warp runs the loop, one lane issues.
-        const uint32_t id0 = idesc<0>();   // N field filled in per MMA: (n >> 3) << 17
-        // A: K chunks kPlane positions apart, or (PAIR) the pair two positions on
-        const uint64_t adesc0 = sdesc(ring, PAIR ? 32 : kPlane * 16, kBX * 16);
-        const uint64_t bdesc0 = sdesc(ws_u, 3 * N * 16, 128);
-        const uint32_t alo0 = uint32_t(adesc0), ahi = uint32_t(adesc0 >> 32);
-        const uint32_t blo0 = uint32_t(bdesc0), bhi = uint32_t(bdesc0 >> 32);
-        uint32_t live[kAccTiles], waited[kAccTiles];   // accf commits / acce completions seen
-        for (int i = 0; i < kAccTiles; ++i) live[i] = waited[i] = 0;
-        uint32_t kp = 0, done = 0;   // planes issued; tiles completed (tile n goes to group n % kEpiGroups)
-        bool ok = true;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const Item it = item_of(a, item);
-            const int L = it.nt;
-            const uint32_t base = kp;
-            for (int u = -1; u <= L; ++u) {
-                const uint32_t p = base + uint32_t(u + 1);
-                const int lo = max(u - 1, 0), hi = min(u + 1, L - 1), nv = hi - lo + 1;
-                const bool first = u + 1 <= L - 1;     // tile u + 1 starts here
-                bool w = role_wait(&full[p % kRing], (p / kRing) & 1u, abort_flag);
-                if (w && first) {
-                    const int c = acc_of(u + 1);
-                    if (waited[c] < live[c]) {          // its last tile's epilogue has read it
-                        w = role_wait(&acce[c], waited[c] & 1u, abort_flag);
-                        ++waited[c];
+        // u − 1, whose accumulators are adjacent.
+        // One elected thread runs the whole loop (waits, MMAs, commits). An MMA of M = 128,
+        // K = 16 takes max(N / 2, 32 + N / 4) cycles, 56 at N = 96 (its operands' shared-memory
+        // reads; the same for every operand layout tried). With the warp converged and an
+        // election per MMA an issue took 52, and the 850 cycles of waits and commits between
+        // planes were not covered by queued MMAs: a hidden layer at 256^3 took 1.26 ms.
+        if (elect_one()) {
+            constexpr uint32_t id0 = kIdesc;
+            // A: K chunks kPlane positions apart, or (PAIR) the pair two positions on
+            const uint64_t adesc0 = sdesc(ring, PAIR ? 32 : kPlane * 16, kBX * 16);
+            const uint64_t bdesc0 = sdesc(ws_u, 3 * N * 16, 128);
+            const uint32_t alo0 = uint32_t(adesc0), ahi = uint32_t(adesc0 >> 32);
+            const uint32_t blo0 = uint32_t(bdesc0), bhi = uint32_t(bdesc0 >> 32);
+            uint32_t used = 0, phase = 0;   // per accumulator: holds an earlier tile; parity of its acce
+            uint32_t kp = 0, done = 0;   // planes issued; tiles completed (tile n goes to group n % kEpiGroups)
+            bool ok = true;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const Item it = item_of(a, item);
+                const int L = it.nt;
+                const uint32_t base = kp;
+                for (int u = -1; u <= L; ++u) {
+                    const uint32_t p = base + uint32_t(u + 1);
+                    const int lo = max(u - 1, 0), hi = min(u + 1, L - 1), nv = hi - lo + 1;
+                    const bool first = u + 1 <= L - 1;     // tile u + 1 starts here
+                    ok = role_wait(&full[p % kRing], (p / kRing) & 1u, abort_flag);
+                    if (ok && first) {
+                        const int c = acc_of(u + 1);
+                        if ((used >> c) & 1u) {             // its last tile's epilogue has read it
+                            ok = role_wait(&acce[c], (phase >> c) & 1u, abort_flag);
+                            phase ^= 1u << c;
+                        }
+                        used |= 1u << c;
+                    }
+                    if (!ok) break;
+                    tc_after_sync();
+                    const uint32_t d0 = tmem + uint32_t(acc_of(hi) * N);
+                    const int b0 = u + 1 - hi;               // weight block (kz) of tile hi
+                    const uint32_t alo = alo0 + (((p % kRing) * kSlot) >> 4);
+                    const uint32_t blo = blo0 + uint32_t(b0 * N);
+                    const uint32_t idv = id0 | (uint32_t(nv * N / 8) << 17);
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                        for (int dx = 0; dx < (PAIR ? 1 : 3); ++dx)
+#pragma unroll
+                            for (int s = 0; s < (PAIR ? 1 : KC / 2); ++s) {
+                                const int sh = PAIR ? dy : dy * 3 + dx;
+                                const uint32_t av = alo + uint32_t(((2 * s * kPlane + dy * kBX + dx) * 16) >> 4);
+                                const uint32_t bv = blo + uint32_t((((sh * KW + 2 * s) * 3 * N) * 16) >> 4);
+                                if (sh == 0 && s == 0 && first) {
+                                    mma_bf16_w(d0, av, ahi, bv, bhi, id0 | (uint32_t(N / 8) << 17), 0u);
+                                    if (nv > 1)
+                                        mma_bf16_w(d0 + N, av, ahi, bv + N, bhi,
+                                                   id0 | (uint32_t((nv - 1) * N / 8) << 17), 1u);
+                                } else {
+                                    mma_bf16_w(d0, av, ahi, bv, bhi, idv, 1u);
+                                }
+                            }
+                    mma_commit(&empty[p % kRing]);
+                    if (u >= 1) {   // tile u − 1 is complete
+                        mma_commit(&accf[(done % kEpiGroups) * kAccTiles + acc_of(u - 1)]);
+                        ++done;
                     }
                 }
-                ok = __all_sync(0xffffffffu, w);
-                if (!ok) break;
-                tc_after_sync();
-                const uint32_t d0 = tmem + uint32_t(acc_of(hi) * N);
-                const int b0 = u + 1 - hi;               // weight block (kz) of tile hi
-                const uint32_t alo = alo0 + (((p % kRing) * kSlot) >> 4);
-                const uint32_t idv = id0 | (uint32_t(nv * N / 8) << 17);
-#pragma unroll
-                for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                    for (int dx = 0; dx < (PAIR ? 1 : 3); ++dx)
-#pragma unroll
-                        for (int s = 0; s < (PAIR ? 1 : KC / 2); ++s) {
-                            const int sh = PAIR ? dy : dy * 3 + dx;
-                            const uint32_t av = alo + uint32_t(((2 * s * kPlane + dy * kBX + dx) * 16) >> 4);
-                            const uint32_t bv =
-                                blo0 + uint32_t((((sh * KW + 2 * s) * 3 * N) * 16) >> 4) + uint32_t(b0 * N);
-                            if (sh == 0 && s == 0 && first) {
-                                mma_bf16_warp(d0, av, ahi, bv, bhi, id0 | (uint32_t(N / 8) << 17), 0u);
-                                if (nv > 1)
-                                    mma_bf16_warp(d0 + N, av, ahi, bv + N, bhi, id0 | (uint32_t((nv - 1) * N / 8) << 17),
-                                                  1u);
-                            } else {
-                                mma_bf16_warp(d0, av, ahi, bv, bhi, idv, 1u);
-                            }
-                        }
-                mma_commit_warp(&empty[p % kRing]);
-                if (u >= 1)   // tile u − 1 is complete
-                    mma_commit_warp(&accf[(done % kEpiGroups) * kAccTiles + acc_of(u - 1)]);
-                __syncwarp();
-                if (u >= 1) {
-                    ++live[acc_of(u - 1)];
-                    ++done;
-                }
+                kp = base + uint32_t(L + 2);
             }
-            if (!ok) break;
-            kp = base + uint32_t(L + 2);
+            // every MMA has completed before the tensor memory is released
+            mma_commit(fin);
+            mbar_wait(fin, 0);
         }
-        // every MMA has completed before the tensor memory is released
-        if (elect_one()) mma_commit(fin);
         __syncwarp();
-        mbar_wait(fin, 0);
     } else {
         // ── epilogue: group g = warp / 4 takes the CTA's tiles n ≡ g (mod kEpiGroups);
         // warp w reads tensor-memory lanes 32·(w % 4) .. +31 ──────────────────────────
@@ -479,8 +471,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int cc = 0; cc < N; ++cc)
             bias[cc] = (MODE != kBackData && cc < (MODE == kLast ? a.nout : a.cout)) ? __ldg(a.bias + cc) : 0.0f;
-        uint32_t uses[kAccTiles];   // this group's earlier tiles per accumulator
-        for (int i = 0; i < kAccTiles; ++i) uses[i] = 0;
+        uint32_t phase = 0;         // per accumulator: parity of this group's next tile in it
         uint32_t n = 0;             // the CTA's tiles so far
         uint32_t kst = 0;           // this group's tiles so far (staging buffer kst % kOutStages)
         const bool ostore = MODE != kLast && a.use_ostore;
@@ -493,13 +484,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int i = 0; i < it.nt; ++i, ++n) {
                 if (int(n % kEpiGroups) != g) continue;
                 const int c = acc_of(i);
-                bool bad = !role_wait(&accf[g * kAccTiles + c], uses[c] & 1u, abort_flag);
+                bool bad = !role_wait(&accf[g * kAccTiles + c], (phase >> c) & 1u, abort_flag);
                 if (ostore) bad = group_bar_or(1 + g, bad);   // the group's barriers stay matched
                 if (bad) {
                     ok = false;
                     break;
                 }
-                ++uses[c];
+                phase ^= 1u << c;
                 tc_after_sync();
                 uint32_t r[N];
 #pragma unroll

@@ -68,6 +68,17 @@ __device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c
                  : "memory");
 }
 
+// One test of the barrier phase with the given parity (the hardware may suspend the
+// thread for a short, bounded time).
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+
 // Waits for the barrier phase with the given parity; false when `limit` SM clock cycles
 // pass without completion (by default 2^31, about a second).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, long long limit = (1LL << 31)) {
