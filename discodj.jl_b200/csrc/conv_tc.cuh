@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // planes were not covered by queued MMAs: a hidden layer at 256^3 took 1.26 ms.
         if (elect_one()) {
             constexpr uint32_t id0 = kIdesc;
+            constexpr int kEarly = PAIR ? 2 : 6;   // shift before which the next plane is waited for
             // A: K chunks kPlane positions apart, or (PAIR) the pair two positions on
             const uint64_t adesc0 = sdesc(ring, PAIR ? 32 : kPlane * 16, kBX * 16);
             const uint64_t bdesc0 = sdesc(ws_u, 3 * N * 16, 128);
@@ -410,20 +411,25 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const Item it = item_of(a, item);
                 const int L = it.nt;
                 const uint32_t base = kp;
-                for (int u = -1; u <= L; ++u) {
+                // plane u has landed, and the accumulator of the tile it starts is free
+                const auto plane_ready = [&](int u) {
                     const uint32_t p = base + uint32_t(u + 1);
-                    const int lo = max(u - 1, 0), hi = min(u + 1, L - 1), nv = hi - lo + 1;
-                    const bool first = u + 1 <= L - 1;     // tile u + 1 starts here
-                    ok = role_wait(&full[p % kRing], (p / kRing) & 1u, abort_flag);
-                    if (ok && first) {
+                    bool r = role_wait(&full[p % kRing], (p / kRing) & 1u, abort_flag);
+                    if (r && u + 1 <= L - 1) {
                         const int c = acc_of(u + 1);
                         if ((used >> c) & 1u) {             // its last tile's epilogue has read it
-                            ok = role_wait(&acce[c], (phase >> c) & 1u, abort_flag);
+                            r = role_wait(&acce[c], (phase >> c) & 1u, abort_flag);
                             phase ^= 1u << c;
                         }
                         used |= 1u << c;
                     }
-                    if (!ok) break;
+                    return r;
+                };
+                ok = plane_ready(-1);
+                for (int u = -1; u <= L && ok; ++u) {
+                    const uint32_t p = base + uint32_t(u + 1);
+                    const int lo = max(u - 1, 0), hi = min(u + 1, L - 1), nv = hi - lo + 1;
+                    const bool first = u + 1 <= L - 1;     // tile u + 1 starts here
                     tc_after_sync();
                     const uint32_t d0 = tmem + uint32_t(acc_of(hi) * N);
                     const int b0 = u + 1 - hi;               // weight block (kz) of tile hi
@@ -437,6 +443,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                             for (int s = 0; s < (PAIR ? 1 : KC / 2); ++s) {
                                 const int sh = PAIR ? dy : dy * 3 + dx;
+                                // the next plane's waits, while the MMAs queued so far keep the
+                                // tensor cores busy (it starts another accumulator than any tile
+                                // that this plane's commits complete)
+                                if (sh == kEarly && s == 0 && u < L) ok = plane_ready(u + 1);
                                 const uint32_t av = alo + uint32_t(((2 * s * kPlane + dy * kBX + dx) * 16) >> 4);
                                 const uint32_t bv = blo + uint32_t((((sh * KW + 2 * s) * 3 * N) * 16) >> 4);
                                 if (sh == 0 && s == 0 && first) {
