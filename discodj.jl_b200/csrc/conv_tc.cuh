@@ -680,6 +680,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == kLoaderWarp) {
         uint32_t kx = 0, ky = 0;
         bool ok = true;
+        // this lane's offsets in a plane whose halo wraps, the same for every plane of a column
+        constexpr int kCopies = (CC * kPlane + 31) / 32;
+        int off[kCopies];
         auto load_plane = [&](const Item& it, int j, bool interior) -> bool {
             const int slot = int(kx % kWRing);
             if (!role_wait(&emptyx[slot], ((kx / kWRing) & 1u) ^ 1u, abort_flag)) return false;
@@ -696,14 +699,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                     mbar_arrive(&fullx[slot]);
                 }
             } else {
-                for (int e = lane; e < CC * kPlane; e += 32) {
-                    const int pos = e / CC, kc = e - pos * CC;
-                    const int by = pos / kBX, bx = pos - by * kBX;
-                    const int gy = wrap(it.y0 - 1 + by, a.res), gx = wrap(it.x0 - 1 + bx, a.res);
-                    const __nv_bfloat16* src = a.X + ((int64_t(gz) * a.res + gy) * a.res + gx) * (CC * 8) + kc * 8;
-                    const uint32_t off = uint32_t((kc * kPlane + pos) * 16);
-                    cp_async16(dst + off, src);
-                    if (mirror) cp_async16(dst2 + off, src);
+                const __nv_bfloat16* const src = a.X + int64_t(gz) * a.res * a.res * (CC * 8);
+#pragma unroll
+                for (int i = 0; i < kCopies; ++i) {
+                    const int e = lane + 32 * i, pos = e / CC, kc = e - pos * CC;
+                    const uint32_t at = uint32_t((kc * kPlane + pos) * 16);
+                    if (e < CC * kPlane) {
+                        cp_async16(dst + at, src + off[i]);
+                        if (mirror) cp_async16(dst2 + at, src + off[i]);
+                    }
                 }
                 cp_async_arrive(&fullx[slot]);
             }
@@ -743,6 +747,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             const Item it = item_of(a, item);
             const bool interior = a.use_tma && it.x0 >= 1 && it.x0 - 1 + kBX <= a.res && it.y0 >= 1 &&
                                   it.y0 - 1 + kBY <= a.res;
+            if (!interior) {
+#pragma unroll
+                for (int i = 0; i < kCopies; ++i) {
+                    const int e = min(lane + 32 * i, CC * kPlane - 1);
+                    const int pos = e / CC, by = pos / kBX, bx = pos - by * kBX;
+                    off[i] = (wrap(it.y0 - 1 + by, a.res) * a.res + wrap(it.x0 - 1 + bx, a.res)) * (CC * 8) +
+                             (e - pos * CC) * 8;
+                }
+            }
             for (int i = 0; i < it.nt && ok; ++i) {
                 if (i == 0) ok = load_plane(it, 0, interior) && load_plane(it, 1, interior);
                 ok = ok && load_plane(it, i + 2, interior) && load_dy(it, i);
@@ -754,35 +767,41 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (uint32_t q = ky > kWY ? ky - kWY : 0; q < ky; ++q) mbar_wait(&fully[q % kWY], (q / kWY) & 1u);
         }
     } else if (warp == kMmaWarp) {
-        const uint32_t id = idesc_mn<N>();
-        // A: M groups (slot, chunk) every 2880 bytes, K groups (tile rows) every 160
-        const uint64_t ad0 = sdesc(ring, kBX * 16, kPlane * 16);
-        // B: N groups every 128 voxels, K groups every 8 voxels
-        const uint64_t bd0 = sdesc(ybuf, 128, 128 * 16);
-        const uint32_t alo0 = uint32_t(ad0), ahi = uint32_t(ad0 >> 32);
-        const uint32_t blo0 = uint32_t(bd0), bhi = uint32_t(bd0 >> 32);
-        uint32_t kx = 0, ky = 0;
-        bool ok = true, first = true;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const Item it = item_of(a, item);
-            const uint32_t base = kx;
-            for (int i = 0; i < it.nt; ++i, ++ky) {
-                bool w = role_wait(&fully[ky % kWY], (ky / kWY) & 1u, abort_flag);
-                for (int j = (i == 0 ? 0 : i + 2); w && j <= i + 2; ++j) {
-                    const uint32_t p = base + uint32_t(j);
-                    w = role_wait(&fullx[p % kWRing], (p / kWRing) & 1u, abort_flag);
-                }
-                ok = __all_sync(0xffffffffu, w);
-                if (!ok) break;
-                tc_after_sync();
-                // window: the slot of plane i (z − 1) and the three after it
-                const uint32_t aw = alo0 + ((((base + i) % kWRing) * kSlot) >> 4);
-                const uint32_t yb = blo0 + (((ky % kWY) * kYBuf) >> 4);
-                if (elect_one()) {
+        if (elect_one()) {   // one thread runs the role, as in k_conv3_tc
+            const uint32_t id = idesc_mn<N>();
+            // A: M groups (slot, chunk) every 2880 bytes, K groups (tile rows) every 160
+            const uint64_t ad0 = sdesc(ring, kBX * 16, kPlane * 16);
+            // B: N groups every 128 voxels, K groups every 8 voxels
+            const uint64_t bd0 = sdesc(ybuf, 128, 128 * 16);
+            const uint32_t alo0 = uint32_t(ad0), ahi = uint32_t(ad0 >> 32);
+            const uint32_t blo0 = uint32_t(bd0), bhi = uint32_t(bd0 >> 32);
+            uint32_t kx = 0, ky = 0;
+            bool ok = true, first = true;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const Item it = item_of(a, item);
+                const uint32_t base = kx;
+                // dY tile `k` and X planes j0 .. j1 of this column have landed
+                const auto ready = [&](uint32_t k, int j0, int j1) {
+                    bool r = role_wait(&fully[k % kWY], (k / kWY) & 1u, abort_flag);
+                    for (int j = j0; r && j <= j1; ++j) {
+                        const uint32_t p = base + uint32_t(j);
+                        r = role_wait(&fullx[p % kWRing], (p / kWRing) & 1u, abort_flag);
+                    }
+                    return r;
+                };
+                ok = ready(ky, 0, 2);
+                for (int i = 0; i < it.nt && ok; ++i, ++ky) {
+                    tc_after_sync();
+                    // window: the slot of plane i (z − 1) and the three after it
+                    const uint32_t aw = alo0 + ((((base + i) % kWRing) * kSlot) >> 4);
+                    const uint32_t yb = blo0 + (((ky % kWY) * kYBuf) >> 4);
 #pragma unroll
                     for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
                         for (int dx = 0; dx < 3; ++dx) {
+                            // the next tile's waits while queued MMAs run (their slots were
+                            // freed by tiles long done)
+                            if (dy == 2 && dx == 1 && i + 1 < it.nt) ok = ready(ky + 1, i + 3, i + 3);
                             const uint32_t d = tmem + uint32_t((dy * 3 + dx) * N);
 #pragma unroll
                             for (int s = 0; s < 8; ++s)
@@ -791,24 +810,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     mma_commit(&emptyx[(base + i) % kWRing]);   // tile i is the last reader of plane i
                     mma_commit(&emptyy[ky % kWY]);
+                    first = false;
                 }
-                __syncwarp();
-                first = false;
-            }
-            if (!ok) break;
-            if (elect_one()) {
+                if (!ok) break;
                 mma_commit(&emptyx[(base + it.nt) % kWRing]);
                 mma_commit(&emptyx[(base + it.nt + 1) % kWRing]);
+                kx = base + it.nt + 2;
             }
-            __syncwarp();
-            kx = base + it.nt + 2;
-        }
-        if (elect_one()) {
             if (ok) mma_commit(accf);
             mma_commit(fin);
+            mbar_wait(fin, 0);
         }
         __syncwarp();
-        mbar_wait(fin, 0);
     } else if (warp < 4) {
         // ── epilogue: warps 0-3, row tid = (window slot q, channel); q = 3 is discarded ──
         const uint32_t lane_base = uint32_t(warp * 32) << 16;
