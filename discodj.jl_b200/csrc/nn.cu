@@ -78,7 +78,8 @@ __device__ __forceinline__ int64_t nbr(int x, int y, int z, int dx, int dy, int 
 // float32 [c][z][y][x] (c < cin) → bf16 [v][cp] (zeros beyond cin, cp a multiple of 8),
 // one voxel per thread. `pair` (cin <= 4, may be null): also the x-pair rows
 // [v][8] = (4 channels of v, 4 channels of its +x neighbour, periodic), the first
-// layer's tensor-core input.
+// layer's tensor-core input. `out` null: the x-pair rows alone (nothing else reads the
+// plain rows outside training; 142 -> 85 us at 256^3).
 __global__ void k_pack(const float* __restrict__ in, int cin, int cp, int res, int64_t nvox,
                        __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ pair) {
     for (int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < nvox; v += int64_t(gridDim.x) * blockDim.x) {
@@ -88,9 +89,9 @@ __global__ void k_pack(const float* __restrict__ in, int cin, int cp, int res, i
 #pragma unroll
         for (int c = 0; c < 8; ++c) f[c] = c < cin ? in[int64_t(c) * nvox + v] : 0.0f;
         uint4* o = reinterpret_cast<uint4*>(out + v * cp);
-        o[0] = make_uint4(djb::conv::pack_bf16(f[0], f[1]), djb::conv::pack_bf16(f[2], f[3]),
+        if (out) o[0] = make_uint4(djb::conv::pack_bf16(f[0], f[1]), djb::conv::pack_bf16(f[2], f[3]),
                           djb::conv::pack_bf16(f[4], f[5]), djb::conv::pack_bf16(f[6], f[7]));
-        for (int c8 = 1; c8 < cp / 8; ++c8) {
+        for (int c8 = 1; out && c8 < cp / 8; ++c8) {
             float h[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) h[j] = c8 * 8 + j < cin ? in[int64_t(c8 * 8 + j) * nvox + v] : 0.0f;
@@ -151,18 +152,38 @@ __global__ void k_bias_out(const float* __restrict__ Y, int n, const float* __re
     }
 }
 
-// dY[v][c] = 2 (out − target) / count and Σ (out − target)² into *sum (double).
-__global__ void k_mse(const float* __restrict__ out, const float* __restrict__ target, int n, int64_t nvox,
-                      double inv_count, float* __restrict__ dY, double* __restrict__ sum) {
+// Gradient of the output mesh as the backward pass reads it, bf16 [v][np] (zeros beyond n),
+// one voxel per thread: 2 (out − target) / count, with Σ (out − target)² into *sum (double);
+// or, with target null, the given gradient `out` itself.
+__global__ void k_out_rows(const float* __restrict__ out, const float* __restrict__ target, int n, int np,
+                           int64_t nvox, double inv_count, __nv_bfloat16* __restrict__ dY, double* __restrict__ sum) {
     __shared__ double part[kNT];
+    const float f = float(2.0 * inv_count);
     double acc = 0.0;
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < nvox * n; t += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t v = t / n;
-        const int c = int(t - v * n);
-        const float d = out[int64_t(c) * nvox + v] - target[int64_t(c) * nvox + v];
-        acc += double(d) * d;
-        dY[t] = float(2.0 * inv_count) * d;
+    for (int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < nvox; v += int64_t(gridDim.x) * blockDim.x) {
+        for (int c8 = 0; c8 < np / 8; ++c8) {
+            float g[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int c = c8 * 8 + j;
+                g[j] = 0.0f;
+                if (c < n) {
+                    const float o = out[int64_t(c) * nvox + v];
+                    if (target) {
+                        const float d = o - target[int64_t(c) * nvox + v];
+                        acc += double(d) * d;
+                        g[j] = f * d;
+                    } else {
+                        g[j] = o;
+                    }
+                }
+            }
+            reinterpret_cast<uint4*>(dY + v * np)[c8] =
+                make_uint4(djb::conv::pack_bf16(g[0], g[1]), djb::conv::pack_bf16(g[2], g[3]),
+                           djb::conv::pack_bf16(g[4], g[5]), djb::conv::pack_bf16(g[6], g[7]));
+        }
     }
+    if (!target) return;
     part[threadIdx.x] = acc;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
@@ -170,15 +191,6 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
         __syncthreads();
     }
     if (threadIdx.x == 0) atomicAdd(sum, part[0]);
-}
-
-// dY[v][c] = dout[c][v]: a given gradient of the output mesh, in the layout k_mse writes.
-__global__ void k_out_grad(const float* __restrict__ dout, int n, int64_t nvox, float* __restrict__ dY) {
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < nvox * n; t += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t v = t / n;
-        const int c = int(t - v * n);
-        dY[t] = dout[int64_t(c) * nvox + v];
-    }
 }
 
 // float32 [v][n] → bf16 [v][np] (zeros beyond n), optionally masked by A > 0 (ReLU backward).
@@ -467,8 +479,8 @@ int launch_tc(djb_nn* h, const djb::conv::Args& a) {
 // The first layer reads the x-pair rows (at most 4 input channels, not the last layer).
 bool use_pair(const djb_nn* h) { return use_tc(h, 0) && h->cin[0] <= 4 && h->cinp[0] == 8 && h->layers > 1; }
 
-// Layer l on the tensor cores: act[l] → act[l + 1] (hidden) or outm (last).
-int conv_tc(djb_nn* h, int l) {
+// Layer l on the tensor cores: act[l] → act[l + 1] (hidden) or the mesh `out` (last).
+int conv_tc(djb_nn* h, int l, float* out) {
     using namespace djb::conv;
     const bool last = (l == h->layers - 1);
     Args a{};
@@ -476,7 +488,7 @@ int conv_tc(djb_nn* h, int l) {
     a.W = h->pb + h->woff[l];
     a.bias = h->p + h->boff[l];
     a.Y = last ? nullptr : h->act[l + 1];
-    a.Yf = last ? h->outm : nullptr;
+    a.Yf = last ? out : nullptr;
     a.res = h->res;
     a.cin = h->cinp[l];
     a.cout = h->coutp[l];
@@ -627,16 +639,19 @@ int ensure_work(djb_nn* h, int res, bool train) {
     return DJB_OK;
 }
 
-// Forward over all voxels: input (float32 mesh, device) → h->outm (float32 mesh).
-int forward(djb_nn* h, const float* in) {
+// Forward over all voxels: input (float32 mesh, device) → `out` (float32 mesh, device; it may
+// be the input, which the first kernel has packed). `train`: keep the input rows that the
+// first layer's weight gradient reads.
+int forward(djb_nn* h, const float* in, float* out, bool train) {
     const int res = h->res;
     const int64_t nvox = int64_t(res) * res * res;
     const float one = 1.0f, zero = 0.0f;
-    k_pack<<<grid_of(nvox), kNT, 0, h->stream>>>(in, h->cin[0], h->cinp[0], res, nvox, h->act[0],
+    k_pack<<<grid_of(nvox), kNT, 0, h->stream>>>(in, h->cin[0], h->cinp[0], res, nvox,
+                                                 train || !use_pair(h) ? h->act[0] : nullptr,
                                                  use_pair(h) ? h->act0p : nullptr);
     for (int l = 0; l < h->layers; ++l) {
             if (use_tc(h, l)) {
-            TRYN(conv_tc(h, l));
+            TRYN(conv_tc(h, l, out));
             continue;
         }
         const int C = h->cinp[l], K = 27 * C;
@@ -650,7 +665,7 @@ int forward(djb_nn* h, const float* in) {
                                     CUDA_R_16BF, h->coutp[l], h->col, CUDA_R_16BF, K, &zero, h->Y, CUDA_R_32F, N,
                                     CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT));
             if (last)
-                k_bias_out<<<grid_of(m * N), kNT, 0, h->stream>>>(h->Y, N, h->p + h->boff[l], nvox, v0, m, h->outm);
+                k_bias_out<<<grid_of(m * N), kNT, 0, h->stream>>>(h->Y, N, h->p + h->boff[l], nvox, v0, m, out);
             else
                 k_bias_act<<<grid_of(m * h->cinp[l + 1]), kNT, 0, h->stream>>>(
                     h->Y, N, h->p + h->boff[l], h->cinp[l + 1], 1, m, h->act[l + 1] + v0 * h->cinp[l + 1]);
@@ -670,16 +685,11 @@ int backward(djb_nn* h, const float* target, double* loss, const float* dout = n
     const int nout = h->cout[L - 1];
     CUDA_TRY(cudaMemsetAsync(h->g, 0, size_t(h->nparam) * sizeof(float), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->lsum, 0, sizeof(double), h->stream));
-    if (target)
-        k_mse<<<grid_of(nvox * nout), kNT, 0, h->stream>>>(h->outm, target, nout, nvox, 1.0 / double(nvox * nout),
-                                                          h->dA, h->lsum);
-    else
-        k_out_grad<<<grid_of(nvox * nout), kNT, 0, h->stream>>>(dout, nout, nvox, h->dA);
     // dY of the last layer (bf16, [v][coutp], no activation)
     __nv_bfloat16* dy = h->dY;
     __nv_bfloat16* dy_next = h->dY2;
-    k_grad_bf16<<<grid_of(nvox * h->coutp[L - 1]), kNT, 0, h->stream>>>(h->dA, nout, h->coutp[L - 1], nullptr, nvox,
-                                                                       dy);
+    k_out_rows<<<grid_of(nvox), kNT, 0, h->stream>>>(target ? h->outm : dout, target, nout, h->coutp[L - 1], nvox,
+                                                    1.0 / double(nvox * nout), dy, h->lsum);
     for (int l = L - 1; l >= 0; --l) {
         const int C = h->cinp[l], K = 27 * C;
         const int N = h->coutp[l];
@@ -879,11 +889,11 @@ int djb_nn_apply(djb_nn* h, const float* in, int32_t res, float* out, int32_t me
     float* din = nullptr;
     bool own_in = false;
     TRYN(stage(h, in, size_t(nvox) * h->cin[0], mem, &din, &own_in));
-    int rc = forward(h, din);
+    const bool direct = mem == DJB_MEM_DEVICE;
+    int rc = forward(h, din, direct ? out : h->outm, false);
     const size_t nout = size_t(nvox) * h->cout[h->layers - 1];
-    if (rc == DJB_OK && cudaMemcpyAsync(out, h->outm, nout * sizeof(float),
-                                        mem == DJB_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
-                                        h->stream) != cudaSuccess)
+    if (rc == DJB_OK && !direct &&
+        cudaMemcpyAsync(out, h->outm, nout * sizeof(float), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
         rc = fail(DJB_ERR_CUDA, "output copy failed");
     if (own_in) cudaFreeAsync(din, h->stream);
     if (rc != DJB_OK) return rc;
@@ -903,7 +913,7 @@ int djb_nn_backward(djb_nn* h, const float* in, const float* target, int32_t res
     bool own_in = false, own_t = false;
     TRYN(stage(h, in, size_t(nvox) * h->cin[0], mem, &din, &own_in));
     int rc = stage(h, target, size_t(nvox) * h->cout[h->layers - 1], mem, &dt, &own_t);
-    if (rc == DJB_OK) rc = forward(h, din);
+    if (rc == DJB_OK) rc = forward(h, din, h->outm, true);
     if (rc == DJB_OK) rc = backward(h, dt, loss);
     if (own_in) cudaFreeAsync(din, h->stream);
     if (own_t) cudaFreeAsync(dt, h->stream);
@@ -924,7 +934,7 @@ int djb_nn_backward_output_grad(djb_nn* h, const float* in, const float* dout, i
     bool own_in = false, own_d = false;
     TRYN(stage(h, in, size_t(nvox) * h->cin[0], mem, &din, &own_in));
     int rc = stage(h, dout, size_t(nvox) * h->cout[h->layers - 1], mem, &dd, &own_d);
-    if (rc == DJB_OK) rc = forward(h, din);
+    if (rc == DJB_OK) rc = forward(h, din, h->outm, true);
     if (rc == DJB_OK) rc = backward(h, nullptr, nullptr, dd);
     if (own_in) cudaFreeAsync(din, h->stream);
     if (own_d) cudaFreeAsync(dd, h->stream);
