@@ -2564,8 +2564,16 @@ int solver_deposit_cic(djb_solver* s, float** mesh_out, int* res, int* pitch, cu
     CUDA_TRY(cudaSetDevice(s->cfg.device));
     CUDA_TRY(cudaMemsetAsync(s->mesh[0], 0, size_t(s->mesh_floats) * sizeof(float), s->stream));
     GroupShifts g{};
-    s->cur_perm = nullptr;  // the P(k) deposit uses Lagrangian tiles
+    // brick-owned, as in the force: the solver's deposit box holds the CIC nodes of the cell
+    // that bins a particle for every assignment order and shift set; without the sort,
+    // Lagrangian tiles
+    s->cur_perm = nullptr;
+    if (s->tiled && s->sorted) {
+        TRY(sort_particles(s, nullptr, 0.0f));
+        s->cur_perm = s->perm;
+    }
     launch_scatter_t<2, 1>(s, nullptr, 0.0f, g, s->mesh[0], nullptr, s->pitch, false);
+    s->cur_perm = nullptr;
     CUDA_TRY(cudaGetLastError());
     *mesh_out = s->mesh[0];
     *res = s->res;

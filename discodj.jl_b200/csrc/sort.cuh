@@ -119,10 +119,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_block(const unsigned* __r
     if (threadIdx.x == kScanThreads - 1) bsum[blockIdx.x] = run;
 }
 
-// Exclusive scan of the block totals, in place (one CTA; nblocks <= kScanThreads * 64).
+// Exclusive scan of the block totals, in place (one CTA; nblocks <= kScanThreads * 64). A
+// thread takes `per` consecutive totals: one at up to 1024 blocks (meshes up to 256^3), where
+// 64 per thread left one thread adding all of them (8 us of every small force).
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(unsigned* __restrict__ bsum, int nblocks) {
     __shared__ unsigned s_warp[kScanThreads / 32];
-    constexpr int per = 64;
+    const int per = (nblocks + kScanThreads - 1) / kScanThreads;
     const int base = threadIdx.x * per;
     unsigned local = 0;
     for (int e = 0; e < per; ++e)
