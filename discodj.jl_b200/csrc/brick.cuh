@@ -186,11 +186,16 @@ __device__ __forceinline__ float brick_fixed_unit(unsigned cnt) {
     return (e - 1 >= 8) ? ldexpf(1.0f, e - 1) : 0.0f;
 }
 
-template <int W, int NS>
+//
+// FIXED: the boxes are added to meshes of 64-bit integers in units of 2^-32 (fx0, fx1: dense
+// [res]^3; mesh0 and mesh1 unused) that k_fixed_to_float turns into floats, so the density
+// does not depend on the order in which three or more bricks add to a node.
+template <int W, int NS, bool FIXED = false>
 __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_SCATTER_BLOCKS) k_scatter_brick(
     const float* __restrict__ psi, const float* __restrict__ q1, int n, int64_t np, float L, int res, int pitch,
     GroupShifts sh, float* __restrict__ mesh0, float* __restrict__ mesh1, int* err, BrickList bl,
-    const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, int tma) {
+    const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, int tma,
+    unsigned long long* __restrict__ fx0 = nullptr, unsigned long long* __restrict__ fx1 = nullptr) {
     constexpr int NB = kScatterBoxes < NS ? kScatterBoxes : NS;  // boxes per particle pass
     extern __shared__ __align__(128) unsigned int sacc[];
     const int b = brick_of_block(bl, blockIdx.x);
@@ -222,14 +227,9 @@ __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_SCATTER_BLOCKS) k_scat
             const unsigned slot = r0 + unsigned((tid & 31) * (kTileThreads / 32) + (tid >> 5));
             if (slot >= cnt) continue;
             const int64_t p = bl.perm[start + slot];
-            float X[3] = {psi[p], psi[p + np], psi[p + 2 * np]};
-            if (q1) {   // else psi holds positions (resampled particle sets)
-                int i, j, k;
-                ld.ijk(p, i, j, k);
-                X[0] += q1[i];
-                X[1] += q1[j];
-                X[2] += q1[k];
-            }
+            int i, j, k;
+            ld.ijk(p, i, j, k);
+            const float X[3] = {psi[p] + q1[i], psi[p + np] + q1[j], psi[p + 2 * np] + q1[k]};
 #pragma unroll 1
             for (int gb = 0; gb < NB; ++gb) {
                 const int g = g0 + gb;
@@ -275,6 +275,22 @@ __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_SCATTER_BLOCKS) k_scat
             }
         }
         __syncthreads();
+        if constexpr (FIXED) {
+#pragma unroll 1
+            for (int gb = 0; gb < NB; ++gb) {
+                unsigned long long* const fx = (g0 + gb == 0) ? fx0 : fx1;
+                const unsigned int* acc = sacc + gb * stride;
+                const unsigned long long unit = fixed ? 4294967296ull / (unsigned long long)(up) : 0ull;
+                for_box_wrapped(box, res, res, false, [&](int so, int64_t go) {
+                    const unsigned v = acc[so];
+                    if (v == 0u) return;
+                    atomicAdd(fx + go, fixed ? v * unit
+                                             : __double2ull_rn(double(__uint_as_float(v)) * 4294967296.0));
+                });
+            }
+            __syncthreads();
+            continue;
+        }
         if (bulk) {
             // fixed point -> float in place, then one bulk reduction per box
             if (fixed)
@@ -312,6 +328,21 @@ __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_SCATTER_BLOCKS) k_scat
             }
             __syncthreads();
         }
+    }
+}
+
+// mesh(x, y, z) = fx · 2^-32 on meshes of row pitch `pitch` (blockIdx.y: the first or the
+// second mesh). The integers are cleared as they are read, for the next deposit.
+__global__ void __launch_bounds__(256) k_fixed_to_float(unsigned long long* __restrict__ fx0,
+                                                        unsigned long long* __restrict__ fx1, int res, int pitch,
+                                                        float* __restrict__ mesh0, float* __restrict__ mesh1) {
+    unsigned long long* const fx = blockIdx.y ? fx1 : fx0;
+    float* const mesh = blockIdx.y ? mesh1 : mesh0;
+    const int total = res * res * res;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const int row = t / res;
+        mesh[int64_t(row) * pitch + (t - row * res)] = __ull2float_rn(fx[t]) * 2.3283064365386963e-10f;
+        fx[t] = 0ull;
     }
 }
 
@@ -518,10 +549,17 @@ __global__ void __launch_bounds__(kTileThreads, DJB_BRICK_GATHER_BLOCKS) k_gathe
 // three fields (rows of sx nodes) are staged together, one bulk tensor copy each where
 // the box does not wrap (`tma` != 0: f is three dense [res]^3 meshes described by
 // tm0..tm2), so each particle's 3 W^3 loads come from shared memory.
+// `kd.mom` != null: the three fields are the whole force of a step; instead of writing it
+// the kernel applies the kick and the second drift (`out` is unused).
+struct KickDrift {
+    float* psi;
+    float* mom;
+    float alpha, beta, dd2;
+};
 template <int W>
 __global__ void __launch_bounds__(kTileThreads, 2) k_interp3_brick(
-    const float* __restrict__ psi, const float* __restrict__ q1, int n, int64_t np, float L, int res,
-    const float* __restrict__ f, float scale, float* __restrict__ out, int* err, BrickList bl, int sx,
+    const float* psi, const float* __restrict__ q1, int n, int64_t np, float L, int res,
+    const float* __restrict__ f, float scale, float* __restrict__ out, KickDrift kd, int* err, BrickList bl, int sx,
     const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
     const __grid_constant__ CUtensorMap tm2, int tma) {
     extern __shared__ __align__(128) float fbox[];
@@ -564,11 +602,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_interp3_brick(
         const int64_t p = bl.perm[start + slot];
         int ijk[3];
         ld.ijk(p, ijk[0], ijk[1], ijk[2]);
-        float w[3][W];
+        float w[3][W], ps[3];
         int d[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const float gc = grid_coord(psi[p + a * np] + q1[ijk[a]], L, resf, err);
+            ps[a] = psi[p + a * np];
+            const float gc = grid_coord(ps[a] + q1[ijk[a]], L, resf, err);
             const int bb = wbase<W>(gc);
 #pragma unroll
             for (int o = 0; o < W; ++o) w[a][o] = wk<W>(fabsf(gc - float(bb + WLo<W>::v + o)));
@@ -598,8 +637,26 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_interp3_brick(
 #pragma unroll
             for (int c = 0; c < 3; ++c) v[c] += w[2][z] * sy[c];
         }
+        if (kd.mom) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) out[p + c * np] = scale * v[c];
+            for (int c = 0; c < 3; ++c) {
+                const float m = kd.alpha * kd.mom[p + c * np] + kd.beta * (scale * v[c]);
+                kd.mom[p + c * np] = m;
+                kd.psi[p + c * np] = ps[c] + kd.dd2 * m;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) out[p + c * np] = scale * v[c];
+        }
+    }
+}
+
+// a[t] = s a[t] + r b[t] over 4·m4 floats (16-byte aligned).
+__global__ void __launch_bounds__(256) k_axpby(float4* __restrict__ a, float s, const float4* __restrict__ b, float r,
+                                               int64_t m4) {
+    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < m4; t += int64_t(gridDim.x) * blockDim.x) {
+        const float4 x = a[t], y = __ldcs(b + t);
+        a[t] = make_float4(s * x.x + r * y.x, s * x.y + r * y.y, s * x.z + r * y.z, s * x.w + r * y.w);
     }
 }
 

@@ -46,8 +46,7 @@ __device__ __forceinline__ uint32_t brick_key(const float X[3], float L, float r
 }
 
 // Applies the first drift Ψ <- Ψ + dd1·Mom when `mom` is given (written back), then
-// bins the particle at X = q + Ψ: key and rank within the key. q1 == null: psi holds the
-// positions themselves.
+// bins the particle at X = q + Ψ: key and rank within the key.
 __global__ void __launch_bounds__(256) k_bin(float* __restrict__ psi, const float* __restrict__ mom,
                                              float dd1, const float* __restrict__ q1, int n, int64_t np,
                                              float L, SortGeom sg, unsigned* __restrict__ count,
@@ -66,11 +65,9 @@ __global__ void __launch_bounds__(256) k_bin(float* __restrict__ psi, const floa
             psi[p + c * np] = X[c];
         }
     }
-    if (q1) {
-        X[0] = X[0] + q1[i];
-        X[1] = X[1] + q1[j];
-        X[2] = X[2] + q1[k];
-    }
+    X[0] = X[0] + q1[i];
+    X[1] = X[1] + q1[j];
+    X[2] = X[2] + q1[k];
     const uint32_t key = brick_key(X, L, float(sg.res), sg, err);
     const unsigned r = atomicAdd(count + key, 1u);
     keyrank[p] = make_uint2(key, r);

@@ -170,3 +170,28 @@ def test_training_gains_over_plain_pm(djb, cosmo, capsys):
               f"P(k) max error k<kNyq/2: plain {ev['pk_max_err_plain']:.4f}, corrected {ev['pk_max_err_corrected']:.4f}")
     assert np.mean(after) < 0.8 * np.mean(before)
     assert ev["pk_max_err_corrected"] < ev["pk_max_err_plain"]
+
+
+@pytest.mark.parametrize("W,grad,n,res,fscale", [(2, 2, 20, 20, 0.3), (3, 4, 17, 32, 4.0), (4, 6, 24, 48, 1e-3)])
+def test_force_and_correction_interpolated_together(djb, W, grad, n, res, fscale):
+    """With one shift and the network on every force, its output and the mesh force are added
+    on the mesh and interpolated once; with another schedule a force call interpolates the
+    correction apart from the potential's gradient. Same sums in another order: 1e-5."""
+    from djb200.nn import ForceNet
+    rng = np.random.default_rng(n)
+    psi = (0.6 * rng.standard_normal((n, n, n, 3))).astype(np.float32)
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=40.0, worder=W, grad_order=grad, deconvolve=True)
+    with ForceNet(layers=3, cin=4, hidden=16, cout=3, seed=3) as net, djb.PMSolver(cfg) as S:
+        S.attach_nn(net, delta_scale=0.5, force_scale=fscale, out_scale=0.2)
+        together = S.acceleration(psi)
+        S.nn_schedule(every=2)
+        apart = S.acceleration(psi)
+        assert np.max(np.abs(together - apart)) < 1e-5 * np.max(np.abs(apart))
+        S.nn_schedule(every=1)
+        S.set_state(psi, psi)
+        S.step(0.0, 0.5, 2.0, 0.25)
+        p, m = S.get_state()
+        m1 = 0.5 * psi + 2.0 * together
+        assert np.max(np.abs(m - m1)) < 2e-5 * np.max(np.abs(m1))
+        assert np.max(np.abs(p - (psi + 0.25 * m1))) < 2e-5 * np.max(np.abs(psi + 0.25 * m1))
+        S.attach_nn(None)

@@ -379,3 +379,35 @@ def test_acceleration_in_place_and_resident_state(djb, grad, aa):
         assert rel(h, djb.logical_view(a).cpu().numpy()) < 1e-5
         p, m = S.get_state(device=True)
         assert torch.equal(p, mom) and torch.equal(m, psi)
+
+
+@pytest.mark.parametrize("W,grad,aa,method,n,res", [(2, 4, 0, "linear", 11, 20), (3, 0, -1, "fourier", 10, 24),
+                                                    (4, 0, 1, "fourier", 12, 36), (4, 6, 2, "linear", 9, 40)])
+def test_resampled_sets_by_brick_match_per_particle_deposit(djb, monkeypatch, W, grad, aa, method, n, res):
+    """The resampled particle sets, sorted and added by brick, against the deposit with one
+    thread per particle (DJB_SORT=0): float32 sums of the same terms (1e-5)."""
+    rng = np.random.default_rng(W + n)
+    psi = (0.8 * rng.standard_normal((n, n, n, 3))).astype(np.float32)
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=30.0, worder=W, grad_order=grad, antialias=aa, n_resample=2,
+                       resampling=method)
+    with djb.PMSolver(cfg) as S:
+        a = S.acceleration(psi)
+    monkeypatch.setenv("DJB_SORT", "0")
+    with djb.PMSolver(cfg) as S:
+        b = S.acceleration(psi)
+    assert rel(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("res,bins,log", [(4, 3, True), (34, 1, False), (66, 40, True), (96, 200, False)])
+def test_shell_sums_sizes_vs_oracle(djb, res, bins, log):
+    """The shell walk at sizes around its 32-wide warps and its segments: mode counts exact,
+    |k| to float64, P(k) to the float32 transform."""
+    from oracle import power as op
+    rng = np.random.default_rng(res)
+    f = rng.standard_normal((res, res, res)).astype(np.float32)
+    k, p, nm = djb.evaluate_power_spectrum(f, 80.0, bins=bins, logarithmic=log)
+    k0, p0, n0 = op.evaluate_power_spectrum(f.astype(np.float64), 80.0, bins=bins, logarithmic=log)
+    assert np.array_equal(nm, n0)
+    assert rel(k, k0) < 1e-13
+    nz = n0 > 0
+    assert np.max(np.abs(p[nz] / p0[nz] - 1)) < 1e-4
