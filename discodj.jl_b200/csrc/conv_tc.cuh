@@ -16,7 +16,7 @@
 //   loader (warp 8): planes into a ring of kRing slots (128-byte aligned), one bulk
 //     tensor copy per plane (5-D map over [z][chunk][y][x][8 channels]) where the halo
 //     does not wrap, else 16-byte cp.async with the periodic wrap; completion on the
-//     slot's `full` barrier.
+//     slot's `full` barrier (cp.async planes: kBehind planes later, see there).
 //   MMA (warp 9; one elected lane runs the loop): per plane, tcgen05.mma of
 //     128 × N·(tiles it feeds) × 16 (bf16 operands, float32 accumulation) per
 //     (dy, dx, K step); commits to the `empty` barrier of the plane and to the `accf`
@@ -54,6 +54,15 @@ constexpr int kPlane = kBX * kBY;                      // 180 positions
 #define DJB_CONV_CTAS 1
 #endif
 constexpr int kRing = DJB_CONV_RING;                   // staged planes
+// Planes copied by cp.async are written through the generic proxy and read by the tensor
+// cores through the async proxy. They are handed over when each lane has seen its own
+// copies land and has fenced the proxies, `kBehind` planes after their issue so that the
+// copies of that many planes stay in flight (forward pass at 256^3 / 96^3: 2.65 to 2.73 ms /
+// 0.27 to 0.31 ms with 1 to 5 planes, 2.83 / 0.31 ms with 6). The loader may block on the slot
+// of plane k - kRing while it holds back planes k - kBehind .. k - 1; that slot is freed by MMAs
+// that wait for planes up to k - kRing + 1, hence the limit.
+constexpr int kBehind = 2;
+static_assert(kBehind >= 1 && kBehind <= kRing - 2, "planes held back must not be ones the ring's oldest slot waits for");
 constexpr int kAccTiles = 16;                          // tile accumulators in tensor memory
 constexpr int kMaxSegment = kAccTiles;                 // z segment length (tiles) at most
 constexpr int kOneCtaSmem = 116 * 1024;                // more than half an SM: one CTA per SM
@@ -113,16 +122,8 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
 // field, (n >> 3) << 17, is filled in per MMA.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(128 >> 4) << 24);
 
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(id), "r"(acc)
-        : "memory");
-}
-
-// The same with the descriptors as (low, high) words: the start address lives in the
-// low word, so per-tap offsets are 32-bit adds.
+// One MMA, descriptors as (low, high) words: the start address lives in the low word, so
+// per-tap offsets are 32-bit adds.
 __device__ __forceinline__ void mma_bf16_w(uint32_t dtmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
                                            uint32_t id, uint32_t acc) {
     asm volatile(
@@ -163,11 +164,11 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Arrives on `bar` when this thread's earlier cp.async copies have landed (the barrier's
-// expected count includes this arrival).
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits until at most N of this thread's cp.async groups are in flight.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -227,6 +228,39 @@ __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, volati
     *abort_flag = 1;
     return false;
 }
+
+// Slots that the loader's lanes fill with cp.async (and stores), on their way to the tensor
+// cores: push() after a slot's copies have been issued, its barrier is arrived on N pushes
+// later, when this lane's copies have landed and the generic and async proxies are fenced;
+// drain() hands over what is still held.
+template <int N>
+struct HandOver {
+    uint64_t* bar[N];   // oldest first; unused entries null
+    __device__ __forceinline__ HandOver() {
+#pragma unroll
+        for (int i = 0; i < N; ++i) bar[i] = nullptr;
+    }
+    __device__ __forceinline__ void push(uint64_t* b) {
+        cp_async_commit();
+        if (bar[0]) {
+            cp_async_wait<N>();
+            fence_proxy_async_smem();
+            mbar_arrive(bar[0]);
+        }
+#pragma unroll
+        for (int i = 0; i + 1 < N; ++i) bar[i] = bar[i + 1];
+        bar[N - 1] = b;
+    }
+    __device__ __forceinline__ void drain() {
+        cp_async_wait<0>();
+        fence_proxy_async_smem();
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (bar[i]) mbar_arrive(bar[i]);
+            bar[i] = nullptr;
+        }
+    }
+};
 
 struct Item {
     int x0, y0, z0, nt;
@@ -339,6 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ── loader ──────────────────────────────────────────────────────────────
         uint32_t k = 0;   // planes issued by this CTA; plane k in slot k % kRing
         bool ok = true;
+        HandOver<kBehind> held;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
             const Item it = item_of(a, item);
             const bool interior = a.use_tma && it.x0 >= 1 && it.x0 - 1 + kBX <= a.res && it.y0 >= 1 &&
@@ -346,7 +381,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             // tiles whose halo wraps: this lane's offsets in a plane, the same for every plane
             constexpr int kCopies = (CC * kPlane + 31) / 32;
             int off[kCopies];
-            if (!interior) {
+            if (interior) {
+                held.drain();
+            } else {
 #pragma unroll
                 for (int i = 0; i < kCopies; ++i) {
                     const int e = min(lane + 32 * i, CC * kPlane - 1);
@@ -377,11 +414,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const int e = lane + 32 * i, pos = e / CC, kc = e - pos * CC;
                         if (e < CC * kPlane) cp_async16(dst + uint32_t((kc * kPlane + pos) * 16), src + off[i]);
                     }
-                    cp_async_arrive(&full[slot]);
+                    held.push(&full[slot]);
                 }
             }
         }
-        cp_async_wait_all();
+        held.drain();
         if (!ok) {
             // bulk copies still in flight land before the CTA ends
             const uint32_t n = k < uint32_t(kRing) ? k : uint32_t(kRing);
@@ -598,6 +635,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 constexpr int kWRing = 8;                  // planes in the ring
 constexpr int kWMirror = 3;                // slots repeated after the ring's end
 constexpr int kWY = 4;                     // dY tile buffers
+// Planes and dY tiles held back (see kBehind). The loader may block on the dY buffer of tile
+// m - kWY while the last planes it issued are m .. m + 2; that buffer is freed by MMAs that
+// wait for plane m - 1, three issues back.
+constexpr int kWBehind = 3;
 
 struct WArgs {
     const __nv_bfloat16* X;   // [nvox][32]
@@ -680,6 +721,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == kLoaderWarp) {
         uint32_t kx = 0, ky = 0;
         bool ok = true;
+        HandOver<kWBehind> held;
         // this lane's offsets in a plane whose halo wraps, the same for every plane of a column
         constexpr int kCopies = (CC * kPlane + 31) / 32;
         int off[kCopies];
@@ -709,7 +751,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         if (mirror) cp_async16(dst2 + at, src + off[i]);
                     }
                 }
-                cp_async_arrive(&fullx[slot]);
+                held.push(&fullx[slot]);
             }
             ++kx;
             return true;
@@ -737,8 +779,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     else
                         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(d), "r"(0) : "memory");
                 }
-                fence_proxy_async_smem();
-                cp_async_arrive(&fully[b]);
+                held.push(&fully[b]);
             }
             ++ky;
             return true;
@@ -747,7 +788,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const Item it = item_of(a, item);
             const bool interior = a.use_tma && it.x0 >= 1 && it.x0 - 1 + kBX <= a.res && it.y0 >= 1 &&
                                   it.y0 - 1 + kBY <= a.res;
-            if (!interior) {
+            if (interior) {
+                held.drain();
+            } else {
 #pragma unroll
                 for (int i = 0; i < kCopies; ++i) {
                     const int e = min(lane + 32 * i, CC * kPlane - 1);
@@ -761,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 ok = ok && load_plane(it, i + 2, interior) && load_dy(it, i);
             }
         }
-        cp_async_wait_all();
+        held.drain();
         if (!ok) {
             for (uint32_t q = kx > kWRing ? kx - kWRing : 0; q < kx; ++q) mbar_wait(&fullx[q % kWRing], (q / kWRing) & 1u);
             for (uint32_t q = ky > kWY ? ky - kWY : 0; q < ky; ++q) mbar_wait(&fully[q % kWY], (q / kWY) & 1u);

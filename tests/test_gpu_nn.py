@@ -162,3 +162,29 @@ def test_tensor_core_backward_matches_im2col(djb, res):
         assert np.max(np.abs(gw - gw_ref)) < 2e-2 * np.max(np.abs(gw_ref))
         gb, gb_ref = g_tc[boff:boff + op], g_ref[boff:boff + op]
         assert np.max(np.abs(gb - gb_ref)) < 2e-2 * np.max(np.abs(gb_ref))
+
+
+@pytest.mark.parametrize("res,hidden", [(9, 8), (17, 32), (18, 16), (33, 24), (100, 32)])
+def test_wrapped_planes_reach_the_tensor_cores(djb, res, hidden):
+    """Planes whose halo wraps are copied by the loader's lanes and handed over some planes
+    later. Sizes: every plane and dY tile copied (9, 17: below the bulk copies' 18), every
+    column wrapped (18, 33), several column segments per CTA of either kind (100); z segments
+    of one tile (17, 33). Against the im2col path: the bf16 rounding of hidden activations
+    whose sums were taken in another order (a plane read early would be wrong by its own size)."""
+    from djb200.nn import ForceNet
+    rng = np.random.default_rng(res)
+    x = rng.standard_normal((4, res, res, res)).astype(np.float32)
+    t = rng.standard_normal((3, res, res, res)).astype(np.float32)
+    with ForceNet(layers=3, cin=4, hidden=hidden, cout=3, seed=res) as net:
+        out = [net.apply(x) for _ in range(3)]
+        net.backward(x, t)
+        g = net.grads()
+        net.set_conv("im2col")
+        ref = net.apply(x)
+        net.backward(x, t)
+        g_ref = net.grads()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    assert np.max(np.abs(out[0] - ref)) < 1e-2 * np.max(np.abs(ref))
+    for (woff, wshape, boff, op, ci, co) in net.layout():
+        n = int(np.prod(wshape))
+        assert np.max(np.abs(g[woff:woff + n] - g_ref[woff:woff + n])) < 2e-2 * np.max(np.abs(g_ref[woff:woff + n]))
