@@ -1817,6 +1817,14 @@ int copy_out(djb_solver* s, float* dst, const float* src, size_t count, int mem)
     return DJB_OK;
 }
 
+// A table of create()'s to the device, on the solver's stream: that stream does not wait for
+// the default stream, on which a plain copy or clear would run. `src` may go on return.
+int upload(djb_solver* s, void* dst, const void* src, size_t bytes) {
+    CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return DJB_OK;
+}
+
 void release(djb_solver* s) {
     if (!s) return;
     int prev = -1;
@@ -1912,10 +1920,10 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
     const double nsets = double(cfg->n_resample) * cfg->n_resample * cfg->n_resample;
     s->s0 = 1.0 / rhomean / nsets / (double(res) * res * res);
     TRY(dmalloc(s, (void**)&s->lapT, sizeof(double) * res));
-    CUDA_TRY(cudaMemcpy(s->lapT, T.data(), sizeof(double) * res, cudaMemcpyHostToDevice));
+    TRY(upload(s, s->lapT, T.data(), sizeof(double) * res));
     if (cfg->deconvolve) {
         TRY(dmalloc(s, (void**)&s->makT, sizeof(double) * res));
-        CUDA_TRY(cudaMemcpy(s->makT, M.data(), sizeof(double) * res, cudaMemcpyHostToDevice));
+        TRY(upload(s, s->makT, M.data(), sizeof(double) * res));
     }
     if (ik) {
         std::vector<float> gh(res / 2 + 1), gf(res);
@@ -1923,14 +1931,14 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
         for (int m = 0; m < res; ++m) gf[m] = (m == res / 2) ? 0.0f : float((m < res / 2 ? m : m - res) * 2 * M_PI / s->L);
         TRY(dmalloc(s, (void**)&s->gh, sizeof(float) * gh.size()));
         TRY(dmalloc(s, (void**)&s->gf, sizeof(float) * gf.size()));
-        CUDA_TRY(cudaMemcpy(s->gh, gh.data(), sizeof(float) * gh.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(cudaMemcpy(s->gf, gf.data(), sizeof(float) * gf.size(), cudaMemcpyHostToDevice));
+        TRY(upload(s, s->gh, gh.data(), sizeof(float) * gh.size()));
+        TRY(upload(s, s->gf, gf.data(), sizeof(float) * gf.size()));
     }
     // lattice coordinates (pm.jl:186): float(i * (L/n))
     std::vector<float> q(s->n);
     for (int i = 0; i < s->n; ++i) q[i] = float(i * (s->L / s->n));
     TRY(dmalloc(s, (void**)&s->q1, sizeof(float) * s->n));
-    CUDA_TRY(cudaMemcpy(s->q1, q.data(), sizeof(float) * s->n, cudaMemcpyHostToDevice));
+    TRY(upload(s, s->q1, q.data(), sizeof(float) * s->n));
 
     const size_t pbytes = size_t(3 * s->np) * sizeof(float);
     TRY(dmalloc(s, (void**)&s->psi, pbytes));
@@ -1975,7 +1983,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             for (int m = 0; m < s->group; ++m) {
                 const size_t bytes = sizeof(unsigned long long) * size_t(s->res) * s->res * s->res;
                 TRY(dmalloc(s, (void**)&s->fx[m], bytes));
-                CUDA_TRY(cudaMemset(s->fx[m], 0, bytes));
+                CUDA_TRY(cudaMemsetAsync(s->fx[m], 0, bytes, s->stream));
             }
         // sorted-order partial sums of the brick interpolation (several shifts);
         // DJB_GATHER_PART=0: through the acceleration array in particle order
@@ -1983,7 +1991,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
         if (s->R > 0 && s->nshift > 1 && !(gp && std::strcmp(gp, "0") == 0))
             TRY(dmalloc(s, (void**)&s->part, 6 * sizeof(float) * size_t(s->np)));
     }
-    CUDA_TRY(cudaMemset(s->err, 0, sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(s->err, 0, sizeof(int), s->stream));
     size_t work = 0;
     TRY(make_plan(&s->r2c, &s->have_r2c, res, CUFFT_R2C, s->stream, &work));
     s->bytes += int64_t(work);
@@ -2024,7 +2032,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             for (int j = 0; j < res; ++j)
                 w[j] = make_float2(float(std::cos(2 * M_PI * j / res)), float(-std::sin(2 * M_PI * j / res)));
             TRY(dmalloc(s, (void**)&s->wN, sizeof(float2) * res));
-            CUDA_TRY(cudaMemcpy(s->wN, w.data(), sizeof(float2) * res, cudaMemcpyHostToDevice));
+            TRY(upload(s, s->wN, w.data(), sizeof(float2) * res));
             if (res == 128) TRY(zpass_attrs<128>());
             if (res == 256) TRY(zpass_attrs<256>());
             if (res == 512) TRY(zpass_attrs<512>());
@@ -2053,7 +2061,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             TRY(dmalloc(s, (void**)&s->bsum_r, sizeof(unsigned) * size_t(s->nscan)));
             TRY(dmalloc(s, (void**)&s->perm_r, sizeof(int) * size_t(s->np)));
             TRY(dmalloc(s, (void**)&s->q0, sizeof(float) * s->n));
-            CUDA_TRY(cudaMemset(s->q0, 0, sizeof(float) * s->n));
+            CUDA_TRY(cudaMemsetAsync(s->q0, 0, sizeof(float) * s->n, s->stream));
         }
         if (cfg->resampling == DJB_RESAMPLE_FOURIER) {
             TRY(dmalloc(s, (void**)&s->psihat, sizeof(float2) * 3 * nspec));
@@ -2076,13 +2084,15 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
                 }
             }
             TRY(dmalloc(s, (void**)&s->phase, sizeof(float2) * h.size()));
-            CUDA_TRY(cudaMemcpy(s->phase, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
+            TRY(upload(s, s->phase, h.data(), sizeof(float2) * h.size()));
             TRY(make_plan(&s->r2c_n, &s->have_r2c_n, n, CUFFT_R2C, s->stream, &work, 3));
             s->bytes += int64_t(work);
             TRY(make_plan(&s->c2r_n, &s->have_c2r_n, n, CUFFT_C2R, s->stream, &work, 3));
             s->bytes += int64_t(work);
         }
     }
+    // the cleared words are there whichever stream the caller sets next
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
     return DJB_OK;
 }
 

@@ -274,3 +274,16 @@ def test_power_spectrum_white_noise_known_answer():
     Vn = L ** 3 / res ** 3
     nz = pk[pk > 0]
     assert 0.5 * Vn < nz.mean() < 2.0 * Vn
+
+
+def test_solver_is_set_up_on_its_own_stream():
+    """The solver's stream does not wait for the default stream (it is created non-blocking),
+    so nothing may be cleared or copied there: a late clear could wipe a first deposit or the
+    zero lattice of the resampled sets. Read from the source; the entry points are not called."""
+    src = open(os.path.join(ROOT, "discodj.jl_b200", "csrc", "solver.cu")).read()
+    assert "cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking)" in src
+    assert not re.search(r"\bcuda(Memset|Memcpy|MemcpyToSymbol)\(", src)
+    create = src[src.index("int create(const djb_pm_config* cfg"):]
+    create = create[:create.index("\n}\n")]
+    last = create.rindex("cudaMemsetAsync(")
+    assert "cudaStreamSynchronize(s->stream)" in create[last:]
