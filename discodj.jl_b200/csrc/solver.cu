@@ -2091,8 +2091,10 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             s->bytes += int64_t(work);
         }
     }
-    // the cleared words are there whichever stream the caller sets next
+    // the cleared words are there whichever stream the caller sets next, and what the caller
+    // queued on the default stream before this call (its inputs, as a rule) has finished
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     return DJB_OK;
 }
 
