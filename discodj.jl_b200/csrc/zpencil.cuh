@@ -32,8 +32,8 @@
 // table of the N roots computed in float64 on the host.
 //
 // Measured per mesh: 1024^3 4.79 ms (8 pencils per CTA on thread pairs) -> 4.19 (this split,
-// loads to registers) -> 3.44 (prefetch) -> 3.24 (twiddles at constant distances, one
-// reciprocal per mode); 512^3 0.45 -> 0.40 -> 0.37 ms, where the 3-D transforms with the
+// loads to registers) -> 3.44 (prefetch) -> 3.21 (twiddles at constant distances, one
+// reciprocal per mode); 512^3 0.45 -> 0.40 -> 0.36 ms, where the 3-D transforms with the
 // multiplication took 0.85 + 0.24 + 0.86 ms and the 2-D ones take 0.53 + 0.54. About 85
 // instructions per mode for 16 bytes moved: the issue slots are half busy (four warps per
 // scheduler, all that 128 registers allow), memory would allow 1.5 ms at 1024^3.
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(ZGeom<N>::kThreads, ZGeom<N>::kBlocks) k_zpass
     fetch(blockIdx.x);
     for (int i = threadIdx.x; i < N; i += G::kThreads) {
         w[i] = wN[(i / M) * (i % M)];   // k1 n2 < N
-        T[i] = kphi.T[i] * kphi.scale;
+        T[i] = kphi.T[i];
         if (kphi.M) D[i] = kphi.M[i];
     }
     __syncthreads();

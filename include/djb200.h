@@ -354,6 +354,10 @@ DJB_API int djb_mesh_deposit3(djb_solver* s, const float* psi, const float* vec,
  * limit_cycles SM cycles (at most 2^31, the kernels' own limit) and *err_word has bit 8
  * set, the kernels' "a wait ran out" flag. No copy is in flight; the device stays usable. */
 DJB_API int djb_selftest_bounded_wait(int32_t device, int32_t arrive, int64_t limit_cycles, int32_t* err_word);
+/* The multiplier of the Poisson solve (inverse Laplacian, deconvolution, mean density) for the
+ * solver's configuration on one plane of modes: out[kz*(res/2+1) + kx] (host) at the given ky,
+ * as the fused z pass (fused = 1) or the general k-space passes (0) evaluate it. */
+DJB_API int djb_selftest_multiplier(djb_solver* s, int32_t ky, int32_t fused, float* out);
 
 /* ── non-allocating shell sums ──────────────────────────────────────────────
  * No counterpart in the reference. For callers that cannot allocate device

@@ -286,3 +286,52 @@ def test_fused_z_pass_sizes_match_3d_transforms(djb, monkeypatch, res, n, W, lap
     with djb.PMSolver(cfg) as B:
         b = B.acceleration(psi)
     assert rel(a, b) < 1e-5
+
+
+def _multiplier64(cfg, ky):
+    """The multiplier on the modes [kz][kx] of one ky in float64, and 0 at the zero mode."""
+    res, L = cfg.res_pm, cfg.boxsize
+    m = res / L
+    i = np.arange(res)
+    k = np.where(i < res // 2, i, i - res) * 2 * np.pi / L
+    t = k / m
+    T = {0: -k * k, 2: -2 * (1 - np.cos(t)) * m * m,
+         4: -(np.cos(2 * t) - 16 * np.cos(t) + 15) / 6 * (m * m),
+         6: -(-2 * np.cos(3 * t) + 27 * np.cos(2 * t) - 270 * np.cos(t) + 245) / 90 * (m * m)}[cfg.lap_order]
+    M = np.sinc(t / (2 * np.pi)) ** (-2.0 * cfg.worder) if cfg.deconvolve else np.ones(res)
+    nh = res // 2 + 1
+    s0 = 1.0 / cfg.n_part ** 3
+    with np.errstate(divide="ignore"):
+        K = s0 / ((T[:nh] + T[ky])[None, :] + T[:, None]) * (M[:nh] * M[ky])[None, :] * M[:, None]
+    if ky == 0:
+        K[0, 0] = 0.0
+    return K
+
+
+@pytest.mark.parametrize("res,L", [(128, 100.0), (256, 3.0e-9), (512, 1000.0), (1024, 2.0e6)])
+def test_fused_multiplier_is_the_float64_quotient(djb, res, L):
+    """The fused z pass' multiplier against float64, mode by mode, for every Laplacian with and
+    without deconvolution and in any unit of length: rounded once, so half a unit in the last
+    place (and 1e-3 of one for the float64 cosines of the finite-difference terms, whose
+    cancellation near k = 0 costs up to 1e5 of their 1e-16). The general passes are compared
+    with the same bound; the two differ only where the quotient lies that close to a tie."""
+    import ctypes as C
+
+    from djb200 import _lib
+    got = [np.empty((res, res // 2 + 1), dtype=np.float32) for _ in range(2)]
+    step = max(1, res // 64)
+    for lap in (0, 2, 4, 6):
+        for dec in (False, True):
+            cfg = djb.PMConfig(res_pm=res, n_part=16, boxsize=L, worder=4, grad_order=4, lap_order=lap,
+                               deconvolve=dec)
+            with djb.PMSolver(cfg) as S:
+                differ = 0
+                for ky in sorted({0, 1, res // 2 - 1, res // 2, res - 1, *range(0, res, step)}):
+                    ref = _multiplier64(cfg, ky)
+                    ulp = np.spacing(np.abs(ref).astype(np.float32)).astype(np.float64)
+                    for fused in (0, 1):
+                        _lib.check(_lib.lib.djb_selftest_multiplier(S.handle, ky, fused,
+                                                                    C.c_void_p(got[fused].ctypes.data)))
+                        assert np.max(np.abs(got[fused] - ref) / ulp) <= 0.5 + 1e-3, (lap, dec, ky, fused)
+                    differ += int(np.sum(got[0] != got[1]))
+                assert differ <= 2, (lap, dec)
