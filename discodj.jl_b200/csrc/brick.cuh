@@ -338,10 +338,11 @@ __global__ void __launch_bounds__(256) k_fixed_to_float(unsigned long long* __re
                                                         float* __restrict__ mesh0, float* __restrict__ mesh1) {
     unsigned long long* const fx = blockIdx.y ? fx1 : fx0;
     float* const mesh = blockIdx.y ? mesh1 : mesh0;
-    const int total = res * res * res;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const int row = t / res;
-        mesh[int64_t(row) * pitch + (t - row * res)] = __ull2float_rn(fx[t]) * 2.3283064365386963e-10f;
+    const int64_t total = int64_t(res) * res * res;
+    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
+         t += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t row = t / res;
+        mesh[row * pitch + (t - row * res)] = __ull2float_rn(fx[t]) * 2.3283064365386963e-10f;
         fx[t] = 0ull;
     }
 }

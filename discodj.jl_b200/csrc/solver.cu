@@ -877,7 +877,7 @@ struct djb_solver {
     // kernels add their boxes to them and fetch their boxes from them with bulk tensor
     // copies described by `tmap_s` (mass-assignment boxes) and `tmap` (interpolation).
     float* phi[kMaxGroup] = {nullptr, nullptr};
-    // fixed-point density meshes of small solvers (k_scatter_brick FIXED), or null
+    // integer density meshes (k_scatter_brick FIXED; DJB_DEPOSIT=integer), or null
     unsigned long long* fx[kMaxGroup] = {nullptr, nullptr};
     CUtensorMap tmap[kMaxGroup];
     CUtensorMap tmap_s[kMaxGroup];
@@ -1139,7 +1139,7 @@ int make_tmap(CUtensorMap* m, const float* base, int res, int sx, int S) {
     return DJB_OK;
 }
 
-// The force's deposit goes through the integer meshes (small meshes, particles in brick order).
+// The force's deposit goes through the integer meshes (asked for, particles in brick order).
 bool fixed_deposit(const djb_solver* s) { return s->fx[0] && s->tiled && s->cur_perm; }
 
 // Mass assignment into m0 (and m1) of row pitch `pitch`; `dense`: m0/m1 are the
@@ -1982,11 +1982,17 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
         TRY(dmalloc(s, (void**)&s->bsum, sizeof(unsigned) * size_t(s->nscan)));
         TRY(dmalloc(s, (void**)&s->keyrank, sizeof(uint2) * size_t(s->np)));
         TRY(dmalloc(s, (void**)&s->perm, sizeof(int) * size_t(s->np)));
-        // Meshes up to 64³: the deposit of a force through 64-bit integers, so that its bits do
-        // not depend on the order in which bricks finish (on larger meshes the float sums of
-        // nodes shared by three or more bricks do). It costs 2 to 8 us of a force of 92 to 152 us;
-        // on larger meshes the scalar 64-bit additions would cost a tenth of it and more.
-        if (s->res <= 64)
+        // DJB_DEPOSIT=integer: the deposit of a force through 64-bit integers, so that its bits
+        // do not depend on the order in which bricks finish, as the float sums of nodes shared
+        // by three or more bricks do. (Resampled sets, the adjoint, P(k) and bricks too dense
+        // for fixed point keep float sums.) For comparing bits, and DJB_GATHER_PART, which
+        // selects between two forms of the interpolation that are to agree in every bit, asks
+        // for it too. Otherwise the float deposit, without scalar 64-bit additions and a pass
+        // over integer meshes: a force of 32³ particles on 64³, PCS, two shifts, 171 us against
+        // 181; CIC, one shift, 93 against 100.
+        const char* dep = std::getenv("DJB_DEPOSIT");
+        const bool integer = dep ? std::strcmp(dep, "integer") == 0 : std::getenv("DJB_GATHER_PART") != nullptr;
+        if (integer)
             for (int m = 0; m < s->group; ++m) {
                 const size_t bytes = sizeof(unsigned long long) * size_t(s->res) * s->res * s->res;
                 TRY(dmalloc(s, (void**)&s->fx[m], bytes));
