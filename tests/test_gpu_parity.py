@@ -436,3 +436,34 @@ def test_integer_deposit_repeats_its_bits_and_matches_float(djb, monkeypatch, W,
         assert all(np.array_equal(o, out[0]) for o in out)
     for o in out:
         assert rel(f, o) < 1e-6
+
+
+@pytest.mark.parametrize("n,res,W,aa", [(128, 32, 2, 0), (128, 64, 4, 2), (128, 128, 3, -1)])
+def test_power_spectrum_of_an_early_state_vs_float64(djb, n, res, W, aa):
+    """P(k) of a slightly perturbed lattice, several particles per cell, against the float64
+    deposit of the same positions. Rounded weights repeat over the lattice, so their errors add
+    up as the displacement's effect does, 0.02 of a cell here. A tile of 256 particles adds its
+    weights in units of 2^-24: off by 2^-25 of 0.02, P by twice that, 3e-6; 2e-6 for the float32
+    node sums and transform. (In bricks of up to 2^18 particles the weights are off by 2^-14.)"""
+    from oracle import nbody as onb
+    from oracle import pm as opm
+    from oracle import power as opw
+    L = 64.0
+    q = np.arange(n) * (L / n)
+    psi = np.zeros((n, n, n, 3), dtype=np.float32)
+    rng = np.random.default_rng(n)
+    for kx, ky, kz in ((1, 0, 0), (0, 2, 1), (3, 1, 2), (2, 2, 5), (7, 3, 1)):
+        phase = 2 * np.pi / L * (kx * q[:, None, None] + ky * q[None, :, None] + kz * q[None, None, :])
+        wave = np.cos(phase + rng.uniform(0, 2 * np.pi)) * (0.02 * L / res)
+        for c, k in enumerate((kx, ky, kz)):
+            psi[..., c] += (k / np.sqrt(kx * kx + ky * ky + kz * kz)) * wave
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=L, worder=W, grad_order=4, antialias=aa)
+    with djb.PMSolver(cfg) as S:
+        S.set_state(psi, psi)
+        k, pk, nm = S.state_power_spectrum(bins=12)
+    X = onb.add_q(psi.astype(np.float64), L).reshape(-1, 3)
+    mesh = opm.pm_scatter(np.zeros((res, res, res)), X, res, L, 2)
+    kr, pkr, nmr = opw.evaluate_power_spectrum(opw.density_contrast(mesh, n), L, bins=12)
+    assert np.array_equal(nm, nmr)
+    live = pkr > 1e-3 * pkr.max()
+    assert np.max(np.abs(pk[live] / pkr[live] - 1)) < 2 * 2.0 ** -25 / 0.02 + 2e-6
