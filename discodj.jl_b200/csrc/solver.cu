@@ -1198,12 +1198,31 @@ void launch_scatter_positions(djb_solver* s, const float* xr, int64_t count, flo
     if (s->W == 4) djb::k_scatter_positions<4><<<b, kThreads, 0, s->stream>>>(xr, count, count, s->Lf, s->res, pitch, mesh, s->err);
 }
 
-// Deposit of n³ given positions (a resampled particle set) into `mesh`: sorted by brick
-// and added by the brick kernel, with sort arrays of its own (the force's order stays valid
-// for its interpolation); without the sort, one thread per particle with float atomics on
-// the mesh. At 96³ particles / 192³ mesh (PCS): see resample_deposit.
+// Whether a resampled particle set is sorted by brick and added by the brick kernel, or added
+// by one thread per particle with float atomics on the mesh. The sort and the launches cost
+// about 25 us a set; what the bricks save grows with the nodes per particle and, for CIC, only
+// with meshes well beyond the L2 (126 MB). A force with 2³ sets, one shift, bricks / threads in
+// ms (early and late times are close; the nearer of the two to a tie):
+//   CIC  64³ on 64³   0.75 / 0.48   256³ on 384³  14.0 / 12.5   256³ on 448³ 15.3 / 15.9
+//        128³ on 512³ 6.1 / 5.5     192³ on 512³   9.1 / 9.6    256³ on 512³ 15.0 / 18.0
+//   TSC  64³ on 64³   0.84 / 0.71    96³ on 96³    1.6 / 1.7    128³ on 128³  2.3 / 3.3
+//        64³ on 256³  1.18 / 0.90    96³ on 384³   3.5 / 3.4    128³ on 384³  4.2 / 4.9
+//   PCS  64³ on 64³   1.37 / 1.20    72³ on 72³    1.26 / 1.47  128³ on 128³  2.7 / 6.2
+//        64³ on 80³   1.01 / 1.14    64³ on 192³   1.00 / 1.16   64³ on 256³  1.32 / 1.23
+// Meshes coarser than the particles keep the threads: bricks of many more than 4096
+// particles add in a coarser fixed-point unit (128³ on 64³, PCS, early: 4.6e-5 from
+// float64 against 3.9e-5; equal at 64³ on 80³ and finer).
+bool sets_by_brick(const djb_solver* s) {
+    if (!(s->tiled && s->sorted) || s->res < s->n || s->res > 3 * s->n) return false;
+    if (s->W == 2) return s->np >= int64_t(192) * 192 * 192 && s->res >= 432;
+    const double work = double(s->np) * s->W * s->W * s->W;   // node additions of a set
+    return work >= 2e7 || (work >= 1.5e7 && 4 * s->res >= 5 * s->n);
+}
+
+// Deposit of n³ given positions (a resampled particle set) into `mesh`, in bricks with sort
+// arrays of its own (the force's order stays valid for its interpolation).
 int scatter_positions(djb_solver* s, const float* xr, float* mesh, int pitch) {
-    if (!(s->tiled && s->sorted && s->perm_r)) {
+    if (!s->perm_r) {
         launch_scatter_positions(s, xr, s->np, mesh, pitch);
         return DJB_OK;
     }
@@ -1223,7 +1242,7 @@ int scatter_positions(djb_solver* s, const float* xr, float* mesh, int pitch) {
 #define DJB_SP(W_)                                                                                              \
     if (s->W == W_)                                                                                             \
         djb::k_scatter_brick<W_, 1><<<nbricks, djb::kTileThreads, scatter_smem(s), s->stream>>>(                 \
-            xr, s->q0, s->n, s->np, s->Lf, s->res, pitch, none, mesh,   nullptr, s->err, bl, s->tmap_s[0],      \
+            xr, s->q0, s->n, s->np, s->Lf, s->res, pitch, none, mesh, nullptr, s->err, bl, s->tmap_s[0],        \
             s->tmap_s[0], tma);
     DJB_SP(2) DJB_SP(3) DJB_SP(4)
 #undef DJB_SP
@@ -2069,7 +2088,7 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
         const int64_t nspec = int64_t(n) * n * nh;
         TRY(dmalloc(s, (void**)&s->rb, sizeof(float) * 3 * size_t(n) * n * (n + 2)));
         TRY(dmalloc(s, (void**)&s->xr, pbytes));
-        if (s->sorted) {
+        if (sets_by_brick(s)) {
             TRY(dmalloc(s, (void**)&s->offset_r, sizeof(unsigned) * size_t(s->nbins)));
             TRY(dmalloc(s, (void**)&s->bsum_r, sizeof(unsigned) * size_t(s->nscan)));
             TRY(dmalloc(s, (void**)&s->perm_r, sizeof(int) * size_t(s->np)));

@@ -384,8 +384,10 @@ def test_acceleration_in_place_and_resident_state(djb, grad, aa):
 @pytest.mark.parametrize("W,grad,aa,method,n,res", [(2, 4, 0, "linear", 11, 20), (3, 0, -1, "fourier", 10, 24),
                                                     (4, 0, 1, "fourier", 12, 36), (4, 6, 2, "linear", 9, 40)])
 def test_resampled_sets_by_brick_match_per_particle_deposit(djb, monkeypatch, W, grad, aa, method, n, res):
-    """The resampled particle sets, sorted and added by brick, against the deposit with one
-    thread per particle (DJB_SORT=0): float32 sums of the same terms (1e-5)."""
+    """A force with resampled particle sets at small sizes, where the particles go by brick and
+    the sets by one thread per particle, against all of them by threads (DJB_SORT=0):
+    float32 sums of the same terms (1e-5). The sizes whose sets go by brick too:
+    test_resampled_sets_deposit_rule."""
     rng = np.random.default_rng(W + n)
     psi = (0.8 * rng.standard_normal((n, n, n, 3))).astype(np.float32)
     cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=30.0, worder=W, grad_order=grad, antialias=aa, n_resample=2,
@@ -467,3 +469,29 @@ def test_power_spectrum_of_an_early_state_vs_float64(djb, n, res, W, aa):
     assert np.array_equal(nm, nmr)
     live = pkr > 1e-3 * pkr.max()
     assert np.max(np.abs(pk[live] / pkr[live] - 1)) < 2 * 2.0 ** -25 / 0.02 + 2e-6
+
+
+@pytest.mark.parametrize("W,grad,aa,method,n,res", [(4, 6, 0, "fourier", 64, 80), (4, 4, -1, "linear", 69, 90),
+                                                    (3, 0, 2, "linear", 92, 96), (3, 4, 0, "fourier", 92, 276),
+                                                    (4, 4, 0, "fourier", 64, 78), (3, 4, 1, "linear", 92, 90),
+                                                    (2, 4, 0, "linear", 192, 432), (2, 4, 0, "linear", 192, 428)])
+def test_resampled_sets_deposit_rule(djb, monkeypatch, W, grad, aa, method, n, res):
+    """Both sides of the rule that sends resampled sets through the brick sort, dense and padded
+    meshes, against the deposits without the sort (DJB_SORT=0): float32 sums of the same
+    terms (1e-5), for a displaced lattice with a collapsed region."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(W + n)
+    L = 30.0
+    psi = 0.3 * (L / n) * torch.randn((3, n, n, n), generator=gen, device="cuda")
+    q = torch.arange(12, device="cuda") * (L / n)
+    for c, shape in enumerate(((1, 1, 12), (1, 12, 1), (12, 1, 1))):
+        psi[c, :12, :12, :12] -= 0.8 * q.view(shape)
+    torch.cuda.synchronize()
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=L, worder=W, grad_order=grad, antialias=aa, n_resample=2,
+                       resampling=method)
+    out = []
+    for sort in ("1", "0"):
+        monkeypatch.setenv("DJB_SORT", sort)
+        with djb.PMSolver(cfg) as S:
+            out.append(S.acceleration(psi).cpu().numpy())
+    assert rel(*out) < 1e-5
