@@ -308,7 +308,7 @@ struct djb_nn {
     __nv_bfloat16* act0p = nullptr;            // [v][8] x-pair rows of the input (use_pair)
     __nv_bfloat16* actw = nullptr;             // [v][32] a narrow layer input widened (training)
     __nv_bfloat16* col = nullptr;              // [chunk][27·Cmax]
-    float* Y = nullptr;                        // [chunk][Nmax] (also dA)
+    float* Y = nullptr;                        // [chunk][Nmax]
     float* dcol = nullptr;                     // [nvox][27·Cmax] (training only)
     float* dA = nullptr;                       // [nvox][Cmax]
     __nv_bfloat16* dY = nullptr;               // [nvox][Cmax]
@@ -606,7 +606,7 @@ int check_derr(djb_nn* h) {
 
 // Work areas for res³ voxels; training needs the whole mesh at once (chunk = nvox).
 // The im2col buffers exist only for layers that do not fit the tensor-core kernels (or
-// every layer after djb_nn_set_conv(h, 1)): col, Y, and dcol when training.
+// every layer after djb_nn_set_conv(h, 1)): col, Y, and dcol and dA when training.
 int ensure_work(djb_nn* h, int res, bool train) {
     const int64_t nvox = int64_t(res) * res * res;
     const bool im2col = any_im2col(h);
@@ -628,7 +628,7 @@ int ensure_work(djb_nn* h, int res, bool train) {
     TRYN(dalloc(h, (void**)&h->lsum, sizeof(double), true));
     if (train) {
         if (im2col) TRYN(dalloc(h, (void**)&h->dcol, size_t(nvox) * 27 * C * sizeof(float), true));
-        TRYN(dalloc(h, (void**)&h->dA, size_t(nvox) * C * sizeof(float), true));
+        if (im2col) TRYN(dalloc(h, (void**)&h->dA, size_t(nvox) * C * sizeof(float), true));
         TRYN(dalloc(h, (void**)&h->dY, size_t(nvox) * C * sizeof(__nv_bfloat16), true));
         TRYN(dalloc(h, (void**)&h->dY2, size_t(nvox) * C * sizeof(__nv_bfloat16), true));
         TRYN(dalloc(h, (void**)&h->actw, size_t(nvox) * 32 * sizeof(__nv_bfloat16), true));

@@ -188,3 +188,28 @@ def test_wrapped_planes_reach_the_tensor_cores(djb, res, hidden):
     for (woff, wshape, boff, op, ci, co) in net.layout():
         n = int(np.prod(wshape))
         assert np.max(np.abs(g[woff:woff + n] - g_ref[woff:woff + n])) < 2e-2 * np.max(np.abs(g_ref[woff:woff + n]))
+
+
+def test_training_work_area_holds_what_the_tensor_core_path_reads(djb):
+    """Per voxel of a 4-layer, 32-channel network: bf16 rows of the input (8) and of three
+    hidden layers, the x-pair rows (8), three float32 outputs, two bf16 gradients of 32
+    channels and the widened input: 428 bytes. A float32 gradient of 32 channels, which only
+    the im2col path reads, would add 128. 8 MB for the parameters and the 2 MB granularity
+    of the device's allocations."""
+    import torch
+    from djb200.nn import ForceNet
+    res = 96
+    x, t = (torch.zeros((c, r, r, r), device="cuda") for c, r in ((4, res), (3, res)))
+    x0, t0 = (torch.zeros((c, 8, 8, 8), device="cuda") for c in (4, 3))
+    with ForceNet(layers=4, cin=4, hidden=32, cout=3, seed=1) as net:
+        net.backward(x0, t0)
+        torch.cuda.synchronize()
+        free0 = torch.cuda.mem_get_info()[0]
+        net.backward(x, t)
+        torch.cuda.synchronize()
+        used = free0 - torch.cuda.mem_get_info()[0]
+        assert used <= 428 * res ** 3 + (8 << 20) + 12 * (2 << 20)
+        net.set_conv("im2col")       # and where a layer does use it, it is there
+        ref = net.backward(x0, t0)
+        net.set_conv("tensor")
+        assert abs(net.backward(x0, t0) - ref) <= 1e-6 * max(ref, 1e-30) + 1e-12
