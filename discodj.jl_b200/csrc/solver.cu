@@ -605,11 +605,12 @@ __global__ void k_output(const float* __restrict__ psi, const float* __restrict_
 // ── sheet resampling (pm.jl:186-234,426-464) ──────────────────────────────────
 // ψ_c = mod(X_c + s_c - q_c + L/2, L) - L/2 with X = q + Psi, written transposed to
 // [i][j][k] (k fastest, row padded to n+2) so that the in-place R2C halves the z
-// axis as the reference's rfft does (pm.jl:430-433). blockIdx.y: the component; `out`
-// holds the three of them `ostride` floats apart.
+// axis as the reference's rfft does (pm.jl:430-433). Components c0 + blockIdx.y; `out`
+// holds them `ostride` floats apart.
 __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restrict__ q1, int n,
-                           int64_t np, float L, Shift3 s, float* __restrict__ out, int64_t ostride) {
-    const int pitch = n + 2, c = blockIdx.y;
+                           int64_t np, float L, Shift3 s, int c0, float* __restrict__ out, int64_t ostride) {
+    const int pitch = n + 2, c = c0 + blockIdx.y;
+    out += blockIdx.y * ostride;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < np;
          t += int64_t(gridDim.x) * blockDim.x) {
         // t enumerates the output in [i][j][k] order (k fastest)
@@ -621,7 +622,7 @@ __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restric
         const int qi = (c == 0) ? ii : (c == 1) ? jj : kk;
         const float X = (psi[p + c * np] + q1[qi]) + sc;
         const float v = jmodf((X - q1[qi]) + L / 2.0f, L) - L / 2.0f;
-        out[c * ostride + (int64_t(ii) * n + jj) * pitch + kk] = v;
+        out[(int64_t(ii) * n + jj) * pitch + kk] = v;
     }
 }
 
@@ -630,7 +631,7 @@ __global__ void k_wrap_psi(const float* __restrict__ psi, const float* __restric
 // kz = n/2 planes are made Hermitian ((H(k) + conj H(-k))/2), which is the value
 // a C2R that ignores the imaginary part of those planes after the full-axis
 // transforms produces from the raw product; it makes the result independent of
-// the C2R implementation. blockIdx.y: the component (three spectra back to back).
+// the C2R implementation. blockIdx.y: the component (spectra back to back).
 __global__ void k_phase(const float2* __restrict__ in, float2* __restrict__ out, int n,
                         const float2* __restrict__ px, const float2* __restrict__ py,
                         const float2* __restrict__ pz, float scale) {
@@ -665,10 +666,11 @@ __global__ void k_phase(const float2* __restrict__ in, float2* __restrict__ out,
 
 // Resampled positions X' = mod(q + ψ' + d·L/n + L, L) for the Fourier method
 // (pm.jl:438-441), ψ' in [i][j][k] padded layout, written to xr (3 blocks of n³,
-// same [i][j][k] order). blockIdx.y: the component.
+// same [i][j][k] order). Components c0 + blockIdx.y, `rstride` floats apart in rb.
 __global__ void k_place(const float* __restrict__ rb, int64_t rstride, const float* __restrict__ q1, int n,
-                        int64_t np, float L, Shift3 shift, float* __restrict__ xr) {
-    const int pitch = n + 2, c = blockIdx.y;
+                        int64_t np, float L, Shift3 shift, int c0, float* __restrict__ xr) {
+    const int pitch = n + 2, c = c0 + blockIdx.y;
+    rb += blockIdx.y * rstride;
     const float shiftc = (c == 0) ? shift.x : (c == 1) ? shift.y : shift.z;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < np;
          t += int64_t(gridDim.x) * blockDim.x) {
@@ -676,7 +678,7 @@ __global__ void k_place(const float* __restrict__ rb, int64_t rstride, const flo
         const int jj = int((t / n) % n);
         const int ii = int(t / (int64_t(n) * n));
         const int qi = (c == 0) ? ii : (c == 1) ? jj : kk;
-        const float v = rb[c * rstride + (int64_t(ii) * n + jj) * pitch + kk];
+        const float v = rb[(int64_t(ii) * n + jj) * pitch + kk];
         xr[t + c * np] = jmodf(((q1[qi] + v) + shiftc) + L, L);
     }
 }
@@ -906,8 +908,9 @@ struct djb_solver {
     float* gf = nullptr;
     // resampling work areas
     float2* psihat = nullptr;   // 3 spectra (n, n, n/2+1)
-    float2* cb = nullptr;       // 3 spectra
-    float* rb = nullptr;        // 3 real n*n*(n+2) arrays
+    int rbatch = 1;             // components that go through the work areas together: 3 or 1
+    float2* cb = nullptr;       // rbatch spectra
+    float* rb = nullptr;        // rbatch real n*n*(n+2) arrays (linear: 3 n³)
     float* xr = nullptr;        // 3*np resampled positions
     float2* phase = nullptr;    // px, py, pz tables (n + n + n/2+1)
     // brick sort of the particles (sort.cuh)
@@ -1366,20 +1369,23 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
     const int64_t nreal = int64_t(n) * n * (n + 2);
     const int nof = int(s->rshifts.size() / 3);
     if (s->cfg.resampling == DJB_RESAMPLE_FOURIER) {
-        // the three components of a set go through each kernel and transform together (a
-        // component alone is launch-sized at the usual 64³-128³ particles)
-        const dim3 gp(unsigned(grid_for(np)), 3), gs(unsigned(grid_for(nspec)), 3);
-        djb::k_wrap_psi<<<gp, kThreads, 0, s->stream>>>(s->psi, s->q1, n, np, s->Lf, sh, s->rb, nreal);
-        CUFFT_TRY(cufftExecR2C(s->r2c_n, s->rb, reinterpret_cast<cufftComplex*>(s->psihat)));
+        const int nb = s->rbatch;
+        const dim3 gp(unsigned(grid_for(np)), unsigned(nb)), gs(unsigned(grid_for(nspec)), unsigned(nb));
+        for (int c = 0; c < 3; c += nb) {
+            djb::k_wrap_psi<<<gp, kThreads, 0, s->stream>>>(s->psi, s->q1, n, np, s->Lf, sh, c, s->rb, nreal);
+            CUFFT_TRY(cufftExecR2C(s->r2c_n, s->rb, reinterpret_cast<cufftComplex*>(s->psihat + c * nspec)));
+        }
         for (int o = 0; o < nof; ++o) {
             const double* d = &s->rshifts[3 * o];
             const float2* px = s->phase + int64_t(o) * (2 * n + nh);
-            djb::k_phase<<<gs, kThreads, 0, s->stream>>>(s->psihat, s->cb, n, px, px + n, px + 2 * n,
-                                                         float(1.0 / (double(n) * n * n)));
-            CUFFT_TRY(cufftExecC2R(s->c2r_n, reinterpret_cast<cufftComplex*>(s->cb), s->rb));
             const Shift3 off{float(d[0] * s->cfg.boxsize / n), float(d[1] * s->cfg.boxsize / n),
                              float(d[2] * s->cfg.boxsize / n)};
-            djb::k_place<<<gp, kThreads, 0, s->stream>>>(s->rb, nreal, s->q1, n, np, s->Lf, off, s->xr);
+            for (int c = 0; c < 3; c += nb) {
+                djb::k_phase<<<gs, kThreads, 0, s->stream>>>(s->psihat + c * nspec, s->cb, n, px, px + n, px + 2 * n,
+                                                             float(1.0 / (double(n) * n * n)));
+                CUFFT_TRY(cufftExecC2R(s->c2r_n, reinterpret_cast<cufftComplex*>(s->cb), s->rb));
+                djb::k_place<<<gp, kThreads, 0, s->stream>>>(s->rb, nreal, s->q1, n, np, s->Lf, off, c, s->xr);
+            }
             TRY(scatter_positions(s, s->xr, mesh, rho_pitch(s)));
         }
     } else {
@@ -1396,8 +1402,6 @@ int resample_deposit(djb_solver* s, int si, float* mesh) {
     return DJB_OK;
 }
 
-// Force evaluation for all shifts; if `step`, fused with the drift/kick/drift.
-// Reads s->psi (and s->mom). Output: s->acc (step == 0) or updated psi/mom.
 // The fused z pass of the Poisson solve on the half spectrum in `mesh`.
 template <int N>
 void launch_zpass_n(djb_solver* s, float* mesh) {
@@ -1443,6 +1447,8 @@ int nn_correction(djb_solver* s, bool whole);
 bool interp3_bricks(const djb_solver* s);
 int interp3(djb_solver* s, const float* f, float scale, float* out, const djb::KickDrift& kd);
 
+// Force evaluation for all shifts; if `step`, fused with the drift/kick/drift.
+// Reads s->psi (and s->mom). Output: s->acc (step == 0) or updated psi/mom.
 int force(djb_solver* s, bool step, double dd1, double alpha, double beta, double dd2) {
     const int nh = s->res / 2 + 1;
     const int64_t nspec = int64_t(s->res) * s->res * nh;
@@ -2086,7 +2092,13 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
     if (resample) {
         const int n = s->n, nh = n / 2 + 1;
         const int64_t nspec = int64_t(n) * n * nh;
-        TRY(dmalloc(s, (void**)&s->rb, sizeof(float) * 3 * size_t(n) * n * (n + 2)));
+        // A component alone is launch-sized at the usual 64³-128³ particles, so the three share
+        // each kernel and transform; at 256³ that still gives 1%, at 320³ one at a time is 0.4%
+        // faster and three would only hold three times the work area and transform space.
+        s->rbatch = s->np <= (int64_t(1) << 24) ? 3 : 1;
+        const bool fourier = cfg->resampling == DJB_RESAMPLE_FOURIER;
+        TRY(dmalloc(s, (void**)&s->rb,
+                    fourier ? sizeof(float) * s->rbatch * size_t(n) * n * (n + 2) : sizeof(float) * 3 * size_t(s->np)));
         TRY(dmalloc(s, (void**)&s->xr, pbytes));
         if (sets_by_brick(s)) {
             TRY(dmalloc(s, (void**)&s->offset_r, sizeof(unsigned) * size_t(s->nbins)));
@@ -2095,9 +2107,9 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             TRY(dmalloc(s, (void**)&s->q0, sizeof(float) * s->n));
             CUDA_TRY(cudaMemsetAsync(s->q0, 0, sizeof(float) * s->n, s->stream));
         }
-        if (cfg->resampling == DJB_RESAMPLE_FOURIER) {
+        if (fourier) {
             TRY(dmalloc(s, (void**)&s->psihat, sizeof(float2) * 3 * nspec));
-            TRY(dmalloc(s, (void**)&s->cb, sizeof(float2) * 3 * nspec));
+            TRY(dmalloc(s, (void**)&s->cb, sizeof(float2) * s->rbatch * nspec));
             // phase tables exp(2πi m d/n) per offset (pm.jl:453-456); full axes hold
             // -n/2 at index n/2, the halved axis m/n for m = 0..n/2
             const int nof = int(s->rshifts.size() / 3);
@@ -2117,9 +2129,9 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
             }
             TRY(dmalloc(s, (void**)&s->phase, sizeof(float2) * h.size()));
             TRY(upload(s, s->phase, h.data(), sizeof(float2) * h.size()));
-            TRY(make_plan(&s->r2c_n, &s->have_r2c_n, n, CUFFT_R2C, s->stream, &work, 3));
+            TRY(make_plan(&s->r2c_n, &s->have_r2c_n, n, CUFFT_R2C, s->stream, &work, s->rbatch));
             s->bytes += int64_t(work);
-            TRY(make_plan(&s->c2r_n, &s->have_c2r_n, n, CUFFT_C2R, s->stream, &work, 3));
+            TRY(make_plan(&s->c2r_n, &s->have_c2r_n, n, CUFFT_C2R, s->stream, &work, s->rbatch));
             s->bytes += int64_t(work);
         }
     }

@@ -495,3 +495,37 @@ def test_resampled_sets_deposit_rule(djb, monkeypatch, W, grad, aa, method, n, r
         with djb.PMSolver(cfg) as S:
             out.append(S.acceleration(psi).cpu().numpy())
     assert rel(*out) < 1e-5
+
+
+@pytest.mark.parametrize("n,res,W", [(24, 48, 3), (256, 80, 2), (258, 80, 2)])
+def test_resampled_sheet_equals_the_finer_lattice(djb, n, res, W):
+    """Fourier resampling of band-limited displacements is exact: the 2^3 sets of n^3 particles
+    are a lattice of (2n)^3, so the forces agree at the particles that both have. Three
+    components together up to 256^3 particles, beyond that one at a time, in less memory than
+    three. Positions differ by roundings of the interpolated displacement (2^-23 of the box
+    side, 2^-23 res = 1e-5 of a cell); 1e-4 of the force of displacements of half a cell."""
+    import torch
+    L = 50.0
+
+    def sheet(m):
+        q = torch.arange(m, device="cuda", dtype=torch.float64) * (2 * np.pi / m)
+        x, y, z = q.view(1, 1, m), q.view(1, m, 1), q.view(m, 1, 1)
+        psi = torch.empty((3, m, m, m), device="cuda")
+        psi[0] = 0.5 * L / res * torch.sin(2 * x + y + 0 * z + 0.3)
+        psi[1] = 0.4 * L / res * torch.cos(3 * z - x + 0 * y)
+        psi[2] = 0.3 * L / res * torch.sin(x + 2 * y - 4 * z)
+        torch.cuda.synchronize()
+        return psi
+
+    cfg = dict(res_pm=res, boxsize=L, worder=W, grad_order=4)
+    with djb.PMSolver(djb.PMConfig(n_part=n, n_resample=2, **cfg)) as S:
+        a, used = S.acceleration(sheet(n)).cpu().numpy(), S.device_bytes
+    with djb.PMSolver(djb.PMConfig(n_part=n, **cfg)) as S:
+        plain = S.device_bytes
+    with djb.PMSolver(djb.PMConfig(n_part=2 * n, **cfg)) as S:
+        b = S.acceleration(sheet(2 * n))[:, ::2, ::2, ::2].cpu().numpy()
+    assert rel(a, b) < 1e-4
+    # positions and spectra of three components, then per component in flight one spectrum, one
+    # real array and the transforms' own space (at most three spectra)
+    per = 4 * n * n * (n + 2)
+    assert used - plain < (6 + 5 * (3 if n <= 256 else 1)) * per + (1 << 20)
