@@ -271,8 +271,9 @@ def test_fused_z_pass_matches_3d_transforms(djb, monkeypatch):
 @pytest.mark.parametrize("res,n,W,lap,dec", [(128, 50, 4, 0, True), (256, 64, 3, 4, False), (512, 48, 2, 0, False),
                                              (512, 70, 4, 6, True)])
 def test_fused_z_pass_sizes_match_3d_transforms(djb, monkeypatch, res, n, W, lap, dec):
-    """The fused z pass at its smaller sizes (one kernel instance each; the last group of 16
-    kx holds one pencil) against the 3-D transforms with the separate multiplication. Both
+    """The fused z pass at its smaller sizes (one kernel instance each; rows of res/2 + 1 pencils,
+    so most tiles of 16 consecutive pencils straddle two ky) against the 3-D transforms with
+    the separate multiplication. Both
     are float32 transforms of the same density: a few 1e-7 per transform, amplified by the
     deconvolution; 1e-5 as at 1024^3."""
     rng = np.random.default_rng(res + n)
