@@ -879,7 +879,8 @@ struct djb_solver {
     // kernels add their boxes to them and fetch their boxes from them with bulk tensor
     // copies described by `tmap_s` (mass-assignment boxes) and `tmap` (interpolation).
     float* phi[kMaxGroup] = {nullptr, nullptr};
-    // integer density meshes (k_scatter_brick FIXED; DJB_DEPOSIT=integer), or null
+    // integer density meshes (k_scatter_brick FIXED), or null; `integer`: for every force
+    bool integer = false;
     unsigned long long* fx[kMaxGroup] = {nullptr, nullptr};
     CUtensorMap tmap[kMaxGroup];
     CUtensorMap tmap_s[kMaxGroup];
@@ -1142,8 +1143,18 @@ int make_tmap(CUtensorMap* m, const float* base, int res, int sx, int S) {
     return DJB_OK;
 }
 
-// The force's deposit goes through the integer meshes (asked for, particles in brick order).
-bool fixed_deposit(const djb_solver* s) { return s->fx[0] && s->tiled && s->cur_perm; }
+// The integer density meshes, cleared (k_fixed_to_float clears them again after each deposit).
+int integer_meshes(djb_solver* s) {
+    const size_t bytes = sizeof(unsigned long long) * size_t(s->res) * s->res * s->res;
+    for (int m = 0; m < s->group && !s->fx[m]; ++m) {
+        TRY(dmalloc(s, (void**)&s->fx[m], bytes));
+        CUDA_TRY(cudaMemsetAsync(s->fx[m], 0, bytes, s->stream));
+    }
+    return DJB_OK;
+}
+
+// The force's deposit goes through the integer meshes (particles in brick order).
+bool fixed_deposit(const djb_solver* s) { return (s->integer || s->nn) && s->fx[0] && s->tiled && s->cur_perm; }
 
 // Mass assignment into m0 (and m1) of row pitch `pitch`; `dense`: m0/m1 are the
 // solver's dense meshes (bulk tensor reductions allowed).
@@ -2014,15 +2025,10 @@ int create(const djb_pm_config* cfg, djb_solver** out) {
         // selects between two forms of the interpolation that are to agree in every bit, asks
         // for it too. Otherwise the float deposit, without scalar 64-bit additions and a pass
         // over integer meshes: a force of 32³ particles on 64³, PCS, two shifts, 171 us against
-        // 181; CIC, one shift, 93 against 100.
+        // 181; CIC, one shift, 93 against 100. (A network on a small mesh: djb_solver_attach_nn.)
         const char* dep = std::getenv("DJB_DEPOSIT");
-        const bool integer = dep ? std::strcmp(dep, "integer") == 0 : std::getenv("DJB_GATHER_PART") != nullptr;
-        if (integer)
-            for (int m = 0; m < s->group; ++m) {
-                const size_t bytes = sizeof(unsigned long long) * size_t(s->res) * s->res * s->res;
-                TRY(dmalloc(s, (void**)&s->fx[m], bytes));
-                CUDA_TRY(cudaMemsetAsync(s->fx[m], 0, bytes, s->stream));
-            }
+        s->integer = dep ? std::strcmp(dep, "integer") == 0 : std::getenv("DJB_GATHER_PART") != nullptr;
+        if (s->integer) TRY(integer_meshes(s));
         // sorted-order partial sums of the brick interpolation (several shifts);
         // DJB_GATHER_PART=0: through the acceleration array in particle order
         const char* gp = std::getenv("DJB_GATHER_PART");
@@ -2362,6 +2368,14 @@ int djb_solver_attach_nn(djb_solver* s, djb_nn* net, double delta_scale, double 
     if (!s->nnf) TRY(dmalloc(s, (void**)&s->nnf, sizeof(float) * size_t(4 * cells)));
     if (!s->nnd) TRY(dmalloc(s, (void**)&s->nnd, sizeof(float) * size_t(3 * cells)));
     if (!s->nnacc) TRY(dmalloc(s, (void**)&s->nnacc, sizeof(float) * size_t(3 * s->np)));
+    // The network rounds its inputs and activations to bf16, so a density that differs in its
+    // last bit (the order of float additions) moves the force by up to 1e-4 of its maximum. On
+    // small meshes, where it costs 3 to 10 us of a corrected force of 240 us and more, the
+    // deposit goes through integers and a corrected force repeats itself.
+    if (s->sorted && s->res <= 64) {
+        TRY(integer_meshes(s));
+        CUDA_TRY(cudaStreamSynchronize(s->stream));   // cleared whichever stream the caller sets next
+    }
     s->nn = net;
     s->nn_in = float(delta_scale);
     s->nn_fin = float(force_scale);

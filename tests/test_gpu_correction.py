@@ -195,3 +195,21 @@ def test_force_and_correction_interpolated_together(djb, W, grad, n, res, fscale
         assert np.max(np.abs(m - m1)) < 2e-5 * np.max(np.abs(m1))
         assert np.max(np.abs(p - (psi + 0.25 * m1))) < 2e-5 * np.max(np.abs(psi + 0.25 * m1))
         S.attach_nn(None)
+
+
+@pytest.mark.parametrize("W,aa,n,res", [(2, 0, 20, 20), (4, 1, 32, 64)])
+def test_corrected_force_on_a_small_mesh_repeats_its_bits(djb, W, aa, n, res):
+    """The network's bf16 roundings would turn a last-bit difference of the density into 1e-4 of
+    the force; up to 64^3 the deposit's bits do not depend on the order of its additions.
+    Without the network the force is the float deposit's again."""
+    from djb200.nn import ForceNet
+    rng = np.random.default_rng(n)
+    psi = (0.6 * rng.standard_normal((n, n, n, 3))).astype(np.float32)
+    cfg = djb.PMConfig(res_pm=res, n_part=n, boxsize=40.0, worder=W, grad_order=4, antialias=aa)
+    with ForceNet(layers=3, cin=4, hidden=16, cout=3, seed=3) as net, djb.PMSolver(cfg) as S:
+        plain = S.acceleration(psi)
+        S.attach_nn(net, delta_scale=0.5, force_scale=0.3, out_scale=0.2)
+        a = [S.acceleration(psi) for _ in range(6)]
+        assert all(np.array_equal(x, a[0]) for x in a)
+        S.attach_nn(None)
+        assert np.max(np.abs(S.acceleration(psi) - plain)) < 1e-6 * np.max(np.abs(plain))
