@@ -1483,9 +1483,14 @@ int force(djb_solver* s, bool step, double dd1, double alpha, double beta, doubl
     // One shift and the network on every force: the mesh force that the network reads as its
     // input and the network's output are added on the mesh and interpolated together, in
     // place of the interpolation from the potential and a second one of the correction
-    // (a corrected step at 256^3 particles and mesh, TSC: 6.61 -> 5.88 ms). Between a schedule's
+    // (a corrected step at 256^3 particles and mesh, TSC: 6.61 -> 5.88 ms). The sum is a pass
+    // over three meshes, which pays while the mesh is at most twice as fine as the particles
+    // (PCS three times): a force of 128^3 particles with a small network, together / apart, CIC
+    // 1.48 / 1.49 ms on 256^3, 2.97 / 2.93 on 320^3, 10.2 / 9.9 on 512^3; PCS 3.24 / 3.40 on
+    // 320^3, 10.9 / 10.9 on 512^3; TSC at 256^3 on 512^3 11.6 / 11.9. Between a schedule's
     // evaluations the particles keep their own correction, so it stays apart there.
     const bool nn_whole = nn_eval && s->nshift == 1 && s->nn_every == 1 &&
+                          s->res <= (s->W == 4 ? 3 : 2) * s->n &&
                           std::fabs(s->nn_fin) > 1e-20f && std::fabs(s->nn_fin) < 1e20f && interp3_bricks(s);
     for (int first = 0; first < s->nshift; first += s->group) {
         const int ns = std::min(s->group, s->nshift - first);

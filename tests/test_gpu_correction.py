@@ -172,7 +172,8 @@ def test_training_gains_over_plain_pm(djb, cosmo, capsys):
     assert ev["pk_max_err_corrected"] < ev["pk_max_err_plain"]
 
 
-@pytest.mark.parametrize("W,grad,n,res,fscale", [(2, 2, 20, 20, 0.3), (3, 4, 17, 32, 4.0), (4, 6, 24, 48, 1e-3)])
+@pytest.mark.parametrize("W,grad,n,res,fscale", [(2, 2, 20, 20, 0.3), (3, 4, 17, 32, 4.0), (4, 6, 24, 48, 1e-3),
+                                                  (4, 6, 16, 48, 0.5), (3, 4, 15, 32, 0.5)])
 def test_force_and_correction_interpolated_together(djb, W, grad, n, res, fscale):
     """With one shift and the network on every force, its output and the mesh force are added
     on the mesh and interpolated once; with another schedule a force call interpolates the
